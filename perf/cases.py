@@ -178,7 +178,17 @@ def _graph(base, cluster, deg, gen):
         nbrs[:, near:] = members[to, torch.randint(0, s - 1, (n, links), generator=gen, device="cuda")]
     rnd = max(1, links // 2) if c > 1 else links
     nbrs[:, deg - rnd:] = torch.randint(0, n, (n, rnd), generator=gen, device="cuda")
-    return nbrs
+    # every list holds distinct ids and not its own node: links that repeat are drawn again
+    own = torch.arange(n, device="cuda")[:, None]
+    while True:
+        ids, at = torch.sort(nbrs, dim=1, stable=True)
+        again = torch.zeros_like(ids, dtype=torch.bool)
+        again[:, 1:] = ids[:, 1:] == ids[:, :-1]
+        again = torch.zeros_like(again).scatter_(1, at, again) | (nbrs == own)
+        bad = int(again.sum())
+        if bad == 0:
+            return nbrs
+        nbrs[again] = torch.randint(0, n, (bad,), generator=gen, device="cuda")
 
 
 def _encode(base):

@@ -36,8 +36,8 @@
 // every acceptance against the reference's test and every logged bound
 // against rp.top() (replay_result, heap_ops.cuh).
 //
-// Visited set: the direct-mapped cache of evaluated ids in shared memory. It
-// may forget an id, never invents one. A forgotten node that is evaluated
+// Visited set: a direct-mapped cache of evaluated ids in shared memory (16-bit
+// tags, VisitedCache below). It may forget an id, never invents one. A forgotten node that is evaluated
 // again has its old distance; if it passes the bound now it was accepted
 // before and is still in the sorted pool with the same id and distance, and
 // it is dropped there.
@@ -56,20 +56,60 @@
 #include "lqg_internal.h"
 #include "lqg_kernels.cuh"
 #include "sq8_batch.cuh"
+#include "sq8_filter.cuh"
 
 namespace lqg {
 
-__host__ __device__ inline size_t batch_warp_bytes(uint32_t dim, uint32_t vbits, uint32_t scap,
-                                                   uint32_t acap) {
-    const size_t dpad = (dim + 15u) & ~15u;
-    return 4 * dpad + 4 * ((size_t)1 << vbits) + kCandBytes + 8 * (size_t)scap + 8 * (size_t)acap;
+// Shared memory of one search warp: byte offsets of its parts.
+struct BatchLayout {
+    uint32_t planes, state, vis, cand, heap, pool, total;
+};
+__host__ __device__ inline BatchLayout batch_layout(uint32_t dim, uint32_t deg, uint32_t vbits,
+                                                    uint32_t scap, uint32_t acap) {
+    BatchLayout L;
+    L.planes = 4u * ((dim + 15u) & ~15u);            // after the query
+    L.state = L.planes + 2u * filter_plane(dim);     // WarpState
+    L.vis = L.state + 32u;                           // visited cache
+    L.cand = L.vis + (4u << vbits);                  // candidate ids, distances
+    L.heap = L.cand + 8u * deg;                      // search heap
+    L.pool = L.heap + 8u * scap;                     // sorted pool: distances, ids
+    L.total = L.pool + 8u * acap;
+    return L;
 }
+
+// The visited cache: 2^(vbits + 1) slots of 16 bits. An id's low B = vbits + 16
+// bits times an odd constant is a bijection on B bits; the top vbits + 1 bits
+// are the slot and the other 15 the tag (0x8000 set: taken), so slot and tag
+// name exactly one id as long as ids are below 2^B (the launcher sees to it).
+// Twice the slots of 32-bit ids in the same bytes: 6 % fewer evaluations at ef
+// 64, 13 % at ef 200 and degree 96.
+struct VisitedCache {
+    uint16_t* s;
+    uint32_t vbits;
+    __device__ __forceinline__ uint32_t key(uint32_t id) const {
+        return (id * 0x9E3779B1u) << (16u - vbits);  // B bits at the top
+    }
+    __device__ __forceinline__ uint16_t* slot(uint32_t k) const { return s + (k >> (31u - vbits)); }
+    __device__ __forceinline__ uint16_t tag(uint32_t k) const {
+        return (uint16_t)((k >> (16u - vbits)) | 0x8000u);
+    }
+};
+
+// Per-query values that are read once or twice per pop: kept in shared memory,
+// so that the search loop's registers hold only what every step needs.
+struct WarpState {
+    float K, st, E;  // the filter's constants (Sq8Filter)
+    uint32_t qi;
+    uint32_t pops, calcs;
+    float smax, n2;  // the filter's per-index sums
+};
+static_assert(sizeof(WarpState) == 32, "BatchLayout reserves 32 bytes");
 
 // After a search, a warp's visited cache, candidates, search heap and sorted
 // pool (contiguous) can hold a result heap of rcap slots.
-__host__ __device__ inline bool batch_replays_in_place(uint32_t vbits, uint32_t scap,
+__host__ __device__ inline bool batch_replays_in_place(uint32_t deg, uint32_t vbits, uint32_t scap,
                                                        uint32_t acap, uint32_t rcap) {
-    return 4 * ((size_t)1 << vbits) + kCandBytes + 8 * (size_t)scap + 8 * (size_t)acap >=
+    return 4 * ((size_t)1 << vbits) + 8 * (size_t)deg + 8 * (size_t)scap + 8 * (size_t)acap >=
            8 * (size_t)rcap;
 }
 
@@ -79,20 +119,19 @@ constexpr uint32_t kPopped = 0x80000000u;  // sorted-pool id flag (ids are < 2^3
 // reference's pushes (every accepted node in order, read from the result log)
 // and pops (each after the logged number of pushes) replayed on an empty
 // heap. Every replayed pop must return the node the lazy search popped there.
-// Returns false, with the heap unusable, when one does not or the heap would
-// outgrow its slots.
-__device__ __forceinline__ bool rebuild_search_heap(const heapops::HeapView sp, uint32_t& sn,
-                                                    uint32_t sp_max, const uint4* rlog,
-                                                    const uint2* plog, uint32_t acc_n,
-                                                    uint32_t pops, int lane) {
+// Returns the heap's size, or kNoId (heap unusable) when one does not or the
+// heap would outgrow its slots. Not inlined: few queries come here, and the
+// search loop has to stay in the instruction cache.
+static __device__ __noinline__ uint32_t rebuild_search_heap(const heapops::HeapView sp, uint32_t sp_max,
+                                                     const uint4* rlog, const uint2* plog,
+                                                     uint32_t acc_n, uint32_t pops, int lane) {
     using namespace heapops;
-    sn = 0;
-    uint32_t i = 0;
+    uint32_t sn = 0, i = 0;
     for (uint32_t j = 0; j <= pops; ++j) {
         const uint2 pj = j < pops ? plog[j] : make_uint2(acc_n, kNoId);
         while (i < pj.x) {
             const uint32_t cnt = min(32u, pj.x - i);
-            if (sn + cnt > sp_max) return false;
+            if (sn + cnt > sp_max) return kNoId;
             const uint4 e = (uint32_t)lane < cnt ? rlog[i + lane] : make_uint4(0, 0, 0, 0);
             for (uint32_t t = 0; t < cnt; ++t) {
                 const uint32_t id = __shfl_sync(kFull, e.x, t);
@@ -102,33 +141,36 @@ __device__ __forceinline__ bool rebuild_search_heap(const heapops::HeapView sp, 
             i += cnt;
         }
         if (j < pops) {
-            if (sn == 0 || sp.get(0).x != pj.y) return false;
+            if (sn == 0 || sp.get(0).x != pj.y) return kNoId;
             warp_pop(sp, sn, lane);
         }
     }
-    return true;
+    return sn;
 }
 
-// Number of entries of the sorted values a[0, n) that are <= y.
+// replay_result out of the search loop's code, as above. (a and ra are
+// __grid_constant__ kernel parameters: nothing is copied.)
+static __device__ __noinline__ bool replay_result_call(const SearchArgs& a, const ReplayArgs& ra,
+                                                       int64_t qi, uint32_t len,
+                                                       const heapops::HeapView rp, int lane) {
+    return replay_result(a, ra, qi, len, rp, lane);
+}
+
+// Number of entries of the sorted values a[0, n) that are <= y: a search
+// without branches or bounds checks (the caller keeps the slots past the last
+// entry at +inf, so n is the array's whole length). One search per lane at the
+// cost of about 35 instructions for any number of members; a rank by ballots,
+// one member after the other, took 26 per member.
 __device__ __forceinline__ uint32_t upper_rank(const float* a, uint32_t n, float y) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] <= y)
-            lo = mid + 1;
-        else
-            hi = mid;
+    const float* p = a;
+#pragma unroll 1
+    while (n > 1) {  // warp-uniform
+        const uint32_t half = n >> 1;
+        if (p[half - 1] <= y) p += half;
+        n -= half;
     }
-    return lo;
+    return (uint32_t)(p - a) + (*p <= y ? 1u : 0u);
 }
-
-// Code words in flight per lane in the distance batches (LW). Up to 256
-// dimensions, 16 keeps the kernel within its 96 registers without spills at
-// degree 32 (32 spilled and ran 13% slower) and larger degrees, which hold
-// more neighbour ids, take 8. Longer rows take 32: a 960-byte row fetched 8
-// words at a time needs dozens of dependent rounds, which costs more than the
-// spills.
-constexpr int batch_load_words(int degw) { return degw == 1 ? 16 : 8; }
 
 // Named barriers of the query-per-block form (barrier 0 is __syncthreads).
 __device__ __forceinline__ void named_bar(uint32_t id, uint32_t threads) {
@@ -138,37 +180,53 @@ constexpr uint32_t kCtaStop = 0xFFFFFFFFu;
 
 // H = 0: one warp per query, blocks of up to 5 query warps. H > 0: one query
 // per block of 1 + H warps (the latency form for small batches): warp 0 runs
-// the search as above, and each expansion's distances are split over all the
-// block's warps, 32 / (H + 1) candidates each, one round of code loads for
-// rows of up to 128 bytes; the other warps only compute distances.
-template <int G, int DEGW, int LW, int H = 0>
-__global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
-    batch_search_kernel(SearchArgs a, ReplayArgs ra) {
-    static_assert(H == 0 || (32 / G) * (H + 1) == 32, "helpers split 32 candidates");
+// the search as above, and each expansion's exact distances are split over all
+// the block's warps, 8 candidates each; the other warps only compute distances.
+//
+// WIDE: rows of kWideDim code bytes or more.
+//
+// What bounds it: instruction issue along one query's dependent steps. A pop
+// costs about 1,000 warp instructions and a lone warp issues one every 2.5
+// cycles, so the code is written for few instructions, short dependent chains
+// and a small instruction footprint (loops over rows and members are not
+// unrolled: unrolled, instruction-cache misses took 20 % of the time).
+// Registers: 96 let 20 warps live on an SM without spills for rows below 256
+// bytes; 24 warps at 80 registers and fewer are slower (spills). Wider rows and
+// the query-per-block form are bound to fewer warps by shared memory, and take
+// 128.
+// Kernel time, before and after the distance bound, the list prefetch, the
+// checked-distinct lists and the 16-bit visited tags (one B200, us):
+//   1M x 128 deg 32 ef 64, 10,000 queries      2,818 -> 2,560
+//   200k x 96 deg 32 ef 100, 37 queries          600 ->   464
+//   100k x 768 deg 64 ef 128, 2,000 queries    4,930 -> 2,470
+//   100k x 960 deg 64 ef 32-512, 2,048        20,550 -> 10,970
+//   100k x 100 deg 96 ef 200, 1,777 queries    3,016 -> 2,334
+template <int DEGW, bool WIDE, int H = 0>
+__global__ void __maxnreg__(WIDE || H ? 128 : 96)
+    batch_search_kernel(const __grid_constant__ SearchArgs a, const __grid_constant__ ReplayArgs ra) {
     using namespace heapops;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
-    const int warp = H ? 0 : (int)(threadIdx.x >> 5);  // the warp's search area
-    const int hw = (int)(threadIdx.x >> 5);            // H > 0: 0 searches, others help
+    const int hw = (int)(threadIdx.x >> 5);  // H > 0: 0 searches, others help
     const uint32_t dim = a.dim;
     const uint32_t dpad = (dim + 15u) & ~15u;
     float* pmin = reinterpret_cast<float*>(smem);
     float* pscale = pmin + dpad;
     const uint32_t vbits = a.vbits;
-    const uint32_t vsize = 1u << vbits;
     const uint32_t acap = ra.acap;
-    unsigned char* wb =
-        smem + 8u * dpad + (size_t)warp * batch_warp_bytes(dim, vbits, ra.scap, acap);
+    const BatchLayout L = batch_layout(dim, 32 * DEGW, vbits, ra.scap, acap);
+    unsigned char* wb = smem + 8u * dpad + (H ? 0u : hw * L.total);
     float* qs = reinterpret_cast<float*>(wb);
-    uint32_t* vis = reinterpret_cast<uint32_t*>(wb + 4u * dpad);
-    uint32_t* cid = vis + vsize;
-    float* cd = reinterpret_cast<float*>(cid + kMaxDeg);
-    uint2* sps = reinterpret_cast<uint2*>(cd + kMaxDeg);
-    float* ad = reinterpret_cast<float*>(sps + ra.scap);  // sorted pool: distances
+    int8_t* planes = reinterpret_cast<int8_t*>(wb + L.planes);
+    volatile WarpState* ws = reinterpret_cast<WarpState*>(wb + L.state);
+    const VisitedCache vis{reinterpret_cast<uint16_t*>(wb + L.vis), vbits};
+    uint32_t* cid = reinterpret_cast<uint32_t*>(wb + L.cand);
+    float* cd = reinterpret_cast<float*>(cid + 32 * DEGW);
+    float* ad = reinterpret_cast<float*>(wb + L.pool);    // sorted pool: distances
     uint32_t* ai = reinterpret_cast<uint32_t*>(ad + acap);  // and ids
-    const size_t gw = (size_t)blockIdx.x * (H ? 1u : (blockDim.x >> 5)) + warp;
-    const HeapView sp{sps, ra.sp_global + gw * ra.gcap, ra.scap};
-    const uint32_t sp_max = ra.scap + ra.gcap;
+    const uint32_t gw = blockIdx.x * (H ? 1u : (blockDim.x >> 5)) + (H ? 0u : hw);
+    const HeapView sp{reinterpret_cast<uint2*>(wb + L.heap), ra.sp_global + (size_t)gw * ra.gcap,
+                      ra.scap};
 
     for (uint32_t i = threadIdx.x; i < dpad; i += blockDim.x) {
         pmin[i] = i < dim ? a.params[2 * i] : 0.f;
@@ -176,9 +234,6 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
     }
     __syncthreads();
 
-    const int g = lane / G, r = lane % G;
-    const uint32_t lt = lanemask_lt();
-    const int64_t mlist = a.nlist ? (int64_t)*a.nlist : a.m;
     const float INF = CUDART_INF_F;
     __shared__ uint32_t s_cmd;   // H > 0: candidates to evaluate, or kCtaStop
     __shared__ uint32_t s_hint;  // H > 0: the first unpopped pool entry's id
@@ -190,9 +245,8 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
                 const uint32_t nc = s_cmd;
                 if (nc == kCtaStop) break;
                 const uint32_t hint = s_hint;
-                for (uint32_t b = 0; b < nc; b += 32)
-                    eval_batch<G, 1, LW, 1>(a, cid, cd, b + (uint32_t)hw * (32 / G), nc, qs, pmin,
-                                            pscale, g, r);
+                for (uint32_t b = 8 * hw; b < nc; b += 32)
+                    eval_few<2>(a, cid, cd, b, nc, qs, pmin, pscale, lane);
                 // The next pop is the first unpopped pool entry or, if one of
                 // this expansion's candidates is accepted below it, that one.
                 // While warp 0 merges, warp 1 reads the pool entry's neighbour
@@ -236,269 +290,230 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
             return;
         }
     }
-    // distances of cid[0, nc) into cd: this warp alone, or split over the block
-    auto eval_all = [&](uint32_t nc, uint32_t hint) {
-        if constexpr (H > 0) {
-            if (lane == 0) {
-                s_cmd = nc;
-                s_hint = hint;
-            }
-            __syncwarp();
-            named_bar(1, kCtaThreads);
-            for (uint32_t b = 0; b < nc; b += 32)
-                eval_batch<G, 1, LW, 1>(a, cid, cd, b, nc, qs, pmin, pscale, g, r);
-            named_bar(2, kCtaThreads);
-        } else {
-            for (uint32_t b = 0; b < nc; b += 32)
-                eval_batch<G, G, LW, 1>(a, cid, cd, b, nc, qs, pmin, pscale, g, r);
+    {
+        float smax, n2;
+        filter_index_sums(pmin, pscale, dim, lane, smax, n2);
+        if (lane == 0) {
+            ws->smax = smax;
+            ws->n2 = n2;
         }
-    };
+        __syncwarp();
+    }
 
     for (;;) {
-        uint32_t slot = 0;
-        if (lane == 0) slot = atomicAdd(a.qhead, 1u);
-        slot = __shfl_sync(kFull, slot, 0);
-        if ((int64_t)slot >= mlist) break;
-        const int64_t qi = a.qlist ? (int64_t)a.qlist[slot] : (int64_t)slot;
-        uint32_t ef = query_ef(a, qi);
-        ef = min(max(ef, 1u), ra.efcap);  // efcap <= acap - 32
-        const float* q = a.queries + (size_t)qi * dim;
-        uint4* rlog = ra.rlog + (size_t)qi * ra.rlog_cap;
-        for (uint32_t i = lane; i < dpad; i += 32) qs[i] = i < dim ? q[i] : 0.f;
-        for (uint32_t i = lane; i < vsize; i += 32) vis[i] = kNoId;
+        uint32_t qi = 0;
+        if (lane == 0) qi = atomicAdd(a.qhead, 1u);
+        qi = __shfl_sync(kFull, qi, 0);
+        if (qi >= (a.nlist ? *a.nlist : (uint32_t)a.m)) break;
+        if (a.qlist) qi = (uint32_t)a.qlist[qi];
+        const uint32_t ef = min(query_ef(a, qi), ra.efcap);  // efcap <= acap - 32
+        {
+            const float* q = a.queries + (size_t)qi * dim;
+#pragma unroll 1
+            for (uint32_t i = lane; i < dpad; i += 32) qs[i] = i < dim ? q[i] : 0.f;
+        }
+#pragma unroll 1
+        for (uint32_t i = 4 * lane; i < (1u << vbits); i += 128)
+            *reinterpret_cast<uint4*>(vis.s + 2 * i) = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+        for (uint32_t i = lane; i < acap; i += 32) ad[i] = INF;  // past the last entry: +inf
         __syncwarp();
-
-        // qg.hpp:305-311: the entry point seeds both pools and is visited
-        const uint32_t ep = a.entry;
-        if (lane == 0) cid[0] = ep;
-        __syncwarp();
-        if constexpr (H > 0)
-            eval_batch<G, 1, LW, 1>(a, cid, cd, 0, 1, qs, pmin, pscale, g, r);
-        else
-            eval_batch<G, G, LW, 1>(a, cid, cd, 0, 1, qs, pmin, pscale, g, r);
-        __syncwarp();
-        const float d0 = cd[0];
-        bool fail = !(d0 < INF);
-        uint32_t acc_n = 1;  // accepted so far (rp.size() = min(acc_n, ef))
-        uint32_t alen = 1;   // sorted-pool entries
-        float lower = d0;
-        uint32_t sn = 1;
-        if (lane == 0) {
-            sp.set(0, make_uint2(ep, __float_as_uint(-d0)));
-            ad[0] = d0;
-            ai[0] = ep;
-            vis[hash_id(ep, vbits)] = ep;
-            rlog[0] = make_uint4(ep, __float_as_uint(d0), __float_as_uint(d0), 0u);
+        {
+            const Sq8Filter f =
+                filter_prepare(qs, pmin, pscale, dim, ws->smax, ws->n2, planes, lane);
+            if (lane == 0) {
+                ws->K = f.K;
+                ws->st = f.st;
+                ws->E = f.E;
+                ws->qi = qi;
+                ws->pops = 0;
+                ws->calcs = 1;
+                // qg.hpp:305-311: the entry point seeds both pools and is
+                // visited; here it is the first round's only candidate
+                cid[0] = a.entry;
+                const uint32_t k = vis.key(a.entry);
+                *vis.slot(k) = vis.tag(k);
+            }
         }
         __syncwarp();
-        uint32_t pops = 0, calcs = 1;
+        bool fail = false;
+        uint32_t acc_n = 0;  // accepted so far (rp.size() = min(acc_n, ef))
+        uint32_t alen = 0;   // sorted-pool entries
+        float lower = INF;
         // Lazy mode: no search heap until a pop meets a tie. The heap's live
         // entries (distance <= lowerBound; the others are never popped) are
         // exactly the unpopped entries of the sorted pool, so while the
         // smallest of them is unique it is the heap's top. `cur` is the first
         // unpopped entry; pops are logged (pushes are the result log) so the
-        // heap can be rebuilt when the smallest distance is shared.
+        // heap can be rebuilt when the smallest distance is shared. sn: the
+        // heap's size.
         bool heap = !ra.lazy;
+        uint32_t sn = 0;
         uint32_t cur = 0;
-        uint2* plg = ra.plog ? ra.plog + (size_t)qi * ra.rlog_cap : nullptr;
-
-        while (!fail) {
-            // qg.hpp:313-318
-            uint32_t u;
-            if (heap) {
-                if (sn == 0) break;
-                const uint2 top = sp.get(0);
-                if (-__uint_as_float(top.y) > lower) break;
-                warp_pop(sp, sn, lane);
-                u = top.x;
-            } else {
-                if (cur >= alen) break;  // nothing live: top > lowerBound or empty
-                uint32_t nxt = alen;
-                for (uint32_t x0 = cur + 1; x0 < alen; x0 += 32) {
-                    const uint32_t x = x0 + lane;
-                    const unsigned um = __ballot_sync(kFull, x < alen && !(ai[x] & kPopped));
-                    if (um) {
-                        nxt = x0 + __ffs(um) - 1;
-                        break;
-                    }
-                }
-                if (nxt < alen && ad[nxt] == ad[cur]) {
-                    // equal smallest distances: the heap layout decides
-                    if (!rebuild_search_heap(sp, sn, sp_max, rlog, plg, acc_n, pops, lane)) {
-                        fail = true;
-                        break;
-                    }
-                    heap = true;
-                    continue;
-                }
-                if (pops >= ra.rlog_cap) {
-                    fail = true;
-                    break;
-                }
-                u = ai[cur];
-                __syncwarp();
-                if (lane == 0) {
-                    ai[cur] = u | kPopped;
-                    plg[pops] = make_uint2(acc_n, u);
-                }
-                __syncwarp();
-                cur = nxt;
-            }
-            ++pops;
-
-            // qg.hpp:320-324: unvisited neighbours in list order
-            uint32_t ncand = 0;
-            const uint32_t* nb = a.nbrs + (size_t)u * a.deg;
-            uint32_t v[DEGW];
+        uint32_t ncand = 1;
+        uint32_t pre = kNoId;  // the node whose list v (and sums sv) hold, or that is prefetched
+        uint32_t v[DEGW];
+        float sv[DEGW];
+        auto load_list = [&]() {
+            const size_t o = (size_t)pre * (32 * DEGW) + lane;
 #pragma unroll
-            for (int w = 0; w < DEGW; ++w) v[w] = __ldg(nb + w * 32 + lane);
-            // A list of degree > 32 spans DEGW words. Repeats inside a word
-            // are caught by match_any; a repeat of an id kept by an earlier
-            // word is caught by the cache, unless another id kept in this
-            // expansion took its slot: then (rare) later words also compare
-            // against the ids already kept, so no node is a candidate twice
-            // (qg.hpp:321). The duplicate check of the acceptance step only
-            // sees the pool from before this expansion.
-            bool lost = false;
+            for (int w = 0; w < DEGW; ++w) v[w] = __ldg(a.nbrs + o + 32 * w);
+            if (a.esum)
 #pragma unroll
-            for (int w = 0; w < DEGW; ++w) {
-                const uint32_t h = hash_id(v[w], vbits);
-                const bool seen = vis[h] == v[w];
-                const unsigned mm = __match_any_sync(kFull, v[w]);
-                bool keep = !seen && (mm & lt) == 0;
-                if (DEGW > 1 && w > 0 && lost && keep)
-                    for (uint32_t j = 0; j < ncand; ++j)
-                        if (cid[j] == v[w]) {
-                            keep = false;
-                            break;
-                        }
-                __syncwarp();
-                if (keep) vis[h] = v[w];
-                const unsigned kb = __ballot_sync(kFull, keep);
-                if (keep) cid[ncand + __popc(kb & lt)] = v[w];
-                ncand += __popc(kb);
-                __syncwarp();
-                if (DEGW > 1 && w + 1 < DEGW) lost = lost || __any_sync(kFull, keep && vis[h] != v[w]);
-            }
+                for (int w = 0; w < DEGW; ++w) sv[w] = __ldg(a.esum + o + 32 * w);
+        };
 
-            // qg.hpp:325-328
+        for (;;) {
+            // qg.hpp:325-328: distances of cid[0, ncand) into cd, by this warp
+            // alone or split over the block
             if constexpr (H > 0) {
-                // the next pop is the first unpopped pool entry or an accepted
-                // candidate of this expansion: ask L2 for the pool entry's list
-                // while the distances are computed
-                if (cur < alen && lane == 0)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.nbrs + (size_t)(ai[cur] & ~kPopped) *
-                                                                         a.deg));
+                if (lane == 0) {
+                    s_cmd = ncand;
+                    s_hint = cur < alen ? (ai[cur] & ~kPopped) : kNoId;
+                }
+                __syncwarp();
+                named_bar(1, kCtaThreads);
+                for (uint32_t b = 0; b < ncand; b += 32)
+                    eval_few<2>(a, cid, cd, b, ncand, qs, pmin, pscale, lane);
+                named_bar(2, kCtaThreads);
+            } else {
+                eval_list(a, cid, cd, ncand, qs, pmin, pscale, lane);
             }
-            eval_all(ncand, cur < alen ? (ai[cur] & ~kPopped) : kNoId);
-            calcs += ncand;
             __syncwarp();
 
             // qg.hpp:329-335: 32 candidates of the list at a time, in order
-#pragma unroll
-            for (int w = 0; w < DEGW; ++w) {
-                const uint32_t c0 = w * 32;
-                if (c0 >= ncand) break;
+#pragma unroll 1
+            for (uint32_t c0 = 0; c0 < ncand; c0 += 32) {
                 const uint32_t c = c0 + lane;
                 const bool valid = c < ncand;
-                const float y = valid ? cd[c] : INF;
+                float y = valid ? cd[c] : INF;
                 const uint32_t id = valid ? cid[c] : kNoId;
-                if (__any_sync(kFull, valid && !(y < INF))) {
+                // a distance that is not finite goes to the exact kernel; once
+                // rp is full it just fails the test, as in the reference
+                if (acc_n < ef && __any_sync(kFull, valid && !(y < INF))) {
                     fail = true;
                     break;
                 }
                 // members: candidates that can pass (all while rp is not full)
                 bool mem = valid && (acc_n < ef || y < lower);
-                uint32_t ub = 0;
-                if (mem) {
-                    ub = upper_rank(ad, alen, y);
-                    // a node the visited cache forgot: still pooled, same distance
-                    for (uint32_t x = ub; x > 0 && ad[x - 1] == y; --x)
-                        if ((ai[x - 1] & ~kPopped) == id) {
-                            mem = false;
-                            break;
-                        }
+                // The next pop is the nearest member if it lies below the first
+                // unpopped entry, else that entry (a tie may decide otherwise):
+                // its list goes into L1 during the merge.
+                {
+                    const float nd = cur < alen ? ad[cur] : INF;
+                    pre = cur < alen ? ai[cur] : kNoId;
+                    const uint32_t yb = mem ? __float_as_uint(y) : 0x7F800000u;
+                    const uint32_t mb = __reduce_min_sync(kFull, yb);
+                    if (mb == 0x7F800000u) continue;  // no member
+                    if (mb < __float_as_uint(nd))
+                        pre = __shfl_sync(kFull, id, __ffs(__ballot_sync(kFull, yb == mb)) - 1);
+                    if (lane < 2 * DEGW) {
+                        const size_t o = (size_t)pre * (32 * DEGW) + 32 * (lane >> 1);
+                        if (!(lane & 1))
+                            prefetch_l1(a.nbrs + o);
+                        else if (a.esum)
+                            prefetch_l1(a.esum + o);
+                    }
                 }
+                const float NaN = __uint_as_float(0x7FC00000u);
+                if (!mem) y = NaN;  // compares false everywhere
+                uint32_t ub = upper_rank(ad, acap, y);
+                // a node the visited cache forgot: still pooled, same distance
+#pragma unroll 1
+                for (uint32_t x = ub; x > 0 && ad[x - 1] == y; --x)
+                    if ((ai[x - 1] & ~kPopped) == id) {
+                        mem = false;
+                        y = NaN;
+                    }
                 const unsigned mmask = __ballot_sync(kFull, mem);
                 if (mmask == 0) continue;
-                // earlier members at or below y
-                uint32_t pc = 0;
-                {
-                    unsigned bm = mmask;
-                    while (bm) {
-                        const int s = __ffs(bm) - 1;
-                        bm &= bm - 1;
-                        const float ys = __shfl_sync(kFull, y, s);
-                        pc += (s < lane && ys <= y) ? 1u : 0u;
-                    }
+                // among the members: pc the earlier ones at or below y, before
+                // the ones placed ahead (equal ones in list order)
+                uint32_t pc = 0, before = 0;
+                const int last = 31 - __clz(mmask);
+#pragma unroll 1
+                for (int s = 0; s <= last; ++s) {
+                    const float ys = __shfl_sync(kFull, y, s);
+                    const bool lo = ys < y, le = ys <= y, early = s < lane;
+                    before += lo || (le && early) ? 1u : 0u;
+                    pc += le && early ? 1u : 0u;
                 }
                 const bool acc = mem && ub + pc < ef;
                 const unsigned am = __ballot_sync(kFull, acc);
                 const uint32_t m = __popc(am);
                 if (m == 0) continue;
-                if (alen + m > acap || acc_n + m > ra.rlog_cap || (heap && sn + m > sp_max)) {
+                if (alen + m > acap || acc_n + m > ra.rlog_cap || (heap && sn + m > ra.scap + ra.gcap)) {
                     fail = true;
                     break;
                 }
-                // merge: accepted j goes after the pooled values <= y_j and the
-                // accepted ones below it (equal ones in list order); pooled
-                // entry x moves up by the number of accepted j with ub_j <= x
-                uint32_t before = 0;
-                uint32_t ubmin = acap;
-                uint32_t shc = 0;   // lazy: accepted ones that go before entry `cur`
-                float pmax = -INF;  // largest accepted value up to this lane
-                {
-                    unsigned bm = am;
-                    while (bm) {
+                if (am != mmask) {  // rare: only the accepted ones count
+                    if (!acc) y = NaN;
+                    before = 0;
+#pragma unroll 1
+                    for (unsigned bm = am; bm; bm &= bm - 1) {
                         const int s = __ffs(bm) - 1;
-                        bm &= bm - 1;
                         const float ys = __shfl_sync(kFull, y, s);
-                        const uint32_t us = __shfl_sync(kFull, ub, s);
-                        before += (ys < y || (ys == y && s < lane)) ? 1u : 0u;
-                        ubmin = min(ubmin, us);
-                        shc += us <= cur ? 1u : 0u;
-                        if (s <= lane) pmax = fmaxf(pmax, ys);
+                        before += ys < y || (ys == y && s < lane) ? 1u : 0u;
                     }
                 }
-                const float old_max = ad[alen - 1];
-                for (int rr = (int)((alen - 1) >> 5); rr >= (int)(ubmin >> 5); --rr) {
+                // merge: accepted j goes after the pooled values <= y_j and the
+                // accepted ones ahead of it. Rows of 32 slots from the top: the
+                // slots taken by accepted ones as a bit mask; every other slot
+                // gets the old entry as many places down as accepted ones lie
+                // below it.
+                const uint32_t pos = ub + before;
+                const uint32_t pmin_new = __reduce_min_sync(kFull, acc ? pos : 0xFFFFFFFFu);
+                const float old_max = alen ? ad[alen - 1] : -INF;
+                uint32_t below = m;  // accepted ones in rows not yet written
+#pragma unroll 1
+                for (int rr = (int)((alen + m - 1) >> 5); rr >= (int)(pmin_new >> 5); --rr) {
+                    const unsigned taken = __reduce_or_sync(
+                        kFull, acc && (int)(pos >> 5) == rr ? 1u << (pos & 31u) : 0u);
+                    below -= __popc(taken);
                     const uint32_t x = (uint32_t)rr * 32 + lane;
-                    const bool have = x < alen && x >= ubmin;
+                    const uint32_t sh = below + __popc(taken & ((1u << lane) - 1u));
+                    const bool mv = sh > 0 && x < alen + m && !((taken >> lane) & 1u);
                     float xd = 0.f;
                     uint32_t xi = 0;
-                    if (have) {
-                        xd = ad[x];
-                        xi = ai[x];
-                    }
-                    uint32_t sh = 0;
-                    unsigned bm = am;
-                    while (bm) {
-                        const int s = __ffs(bm) - 1;
-                        bm &= bm - 1;
-                        sh += __shfl_sync(kFull, ub, s) <= x ? 1u : 0u;
+                    if (mv) {
+                        xd = ad[x - sh];
+                        xi = ai[x - sh];
                     }
                     __syncwarp();
-                    if (have) {
-                        ad[x + sh] = xd;
-                        ai[x + sh] = xi;
+                    if (mv) {
+                        ad[x] = xd;
+                        ai[x] = xi;
                     }
                     __syncwarp();
                 }
                 if (acc) {
-                    ad[ub + before] = y;
-                    ai[ub + before] = id;
+                    ad[pos] = y;
+                    ai[pos] = id;
                 }
                 __syncwarp();
                 // the first unpopped entry: the one at `cur` moved up, or an
                 // accepted one placed before it
-                cur = min(cur + shc, __reduce_min_sync(kFull, acc ? ub + before : 0xFFFFFFFFu));
+                cur = min(cur + __popc(__ballot_sync(kFull, acc && ub <= cur)), pmin_new);
                 alen += m;
                 const uint32_t acc_new = acc_n + m;
                 const float lf = ad[min(acc_new, ef) - 1];
-                // the bound after the t-th accepted (qg.hpp:333-334), logged
-                const uint32_t t = __popc(am & lt) + 1;
+                // the bound after the t-th accepted (qg.hpp:333-334), logged:
+                // read off the merged pool once rp is full, before that the
+                // largest value so far
+                const uint32_t t = __popc(am & ((1u << lane) - 1u)) + 1;
+                float lb = 0.f;
+                if (acc_n + 1 < ef) {
+                    float pmax = acc ? y : -INF;  // inclusive prefix maximum
+#pragma unroll 1
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const float v = __shfl_up_sync(kFull, pmax, o);
+                        if (lane >= o) pmax = fmaxf(pmax, v);
+                    }
+                    lb = fmaxf(old_max, pmax);
+                }
                 if (acc) {
-                    const float lb = acc_n + t >= ef ? ad[ef - 1 + m - t] : fmaxf(old_max, pmax);
+                    if (acc_n + t >= ef) lb = ad[ef - 1 + m - t];
+                    uint4* rlog = ra.rlog + (size_t)ws->qi * ra.rlog_cap;
                     rlog[acc_n + t - 1] =
                         make_uint4(id, __float_as_uint(y), __float_as_uint(lb), 0u);
                 }
@@ -506,12 +521,18 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
                 // bound stay in the sorted pool
                 if (acc_new > ef) {
                     uint32_t keep = ef;
-                    for (uint32_t x0 = ef; x0 < alen; x0 += 32) {
-                        const uint32_t x = x0 + lane;
-                        const unsigned em = __ballot_sync(kFull, x < alen && ad[x] == lf);
-                        keep += __popc(em);
-                        if (em != kFull) break;
+                    if (ad[ef] == lf) {  // (slots past the last entry hold +inf)
+#pragma unroll 1
+                        for (uint32_t x0 = ef; x0 < alen; x0 += 32) {
+                            const uint32_t x = x0 + lane;
+                            const unsigned em = __ballot_sync(kFull, x < alen && ad[x] == lf);
+                            keep += __popc(em);
+                            if (em != kFull) break;
+                        }
                     }
+                    __syncwarp();
+#pragma unroll 1
+                    for (uint32_t x = keep + lane; x < alen; x += 32) ad[x] = INF;
                     alen = keep;
                 }
                 lower = lf;
@@ -527,8 +548,128 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
                 }
                 __syncwarp();
             }
+            if (fail) break;
+
+            // qg.hpp:313-318
+            uint32_t u, nxt = alen;
+            if (!heap) {
+                if (cur >= alen) break;  // nothing live: top > lowerBound or empty
+                pre = ai[cur];           // in a tie, another node may be popped
+                load_list();
+#pragma unroll 1
+                for (uint32_t x0 = cur + 1; x0 < alen; x0 += 32) {
+                    const uint32_t x = x0 + lane;
+                    const unsigned um = __ballot_sync(kFull, x < alen && !(ai[x] & kPopped));
+                    if (um) {
+                        nxt = x0 + __ffs(um) - 1;
+                        break;
+                    }
+                }
+                if (nxt < alen && ad[nxt] == ad[cur]) {
+                    // equal smallest distances: the heap layout decides
+                    const size_t lo = (size_t)ws->qi * ra.rlog_cap;
+                    sn = rebuild_search_heap(sp, ra.scap + ra.gcap, ra.rlog + lo, ra.plog + lo,
+                                             acc_n, ws->pops, lane);
+                    if (sn == kNoId) {
+                        fail = true;
+                        break;
+                    }
+                    heap = true;
+                }
+            }
+            if (heap) {
+                if (sn == 0) break;
+                const uint2 top = sp.get(0);
+                if (-__uint_as_float(top.y) > lower) break;
+                warp_pop(sp, sn, lane);
+                u = top.x;
+            } else {
+                u = pre;
+                __syncwarp();
+                if (lane == 0) {
+                    ai[cur] = u | kPopped;
+                    // (pops < accepted nodes <= rlog_cap)
+                    ra.plog[(size_t)ws->qi * ra.rlog_cap + ws->pops] = make_uint2(acc_n, u);
+                }
+                cur = nxt;
+            }
+            if (lane == 0) ws->pops = ws->pops + 1;
+            __syncwarp();
+
+            // qg.hpp:320-324: unvisited neighbours in list order
+            if (u != pre || heap) {
+                pre = u;
+                load_list();
+            }
+            ncand = 0;
+            // A list of degree > 32 spans DEGW words. Where the index's lists
+            // may repeat an id (SearchArgs::distinct): repeats inside a word
+            // are caught by match_any (about 400 cycles); a repeat of an id
+            // kept by an earlier word is caught by the cache, unless another
+            // id kept in this expansion (in its own word or a later one) took
+            // its slot: then (rare) later words also compare against the ids
+            // already kept, so no node is a candidate twice (qg.hpp:321). The
+            // duplicate check of the acceptance step only sees the pool from
+            // before these candidates.
+            bool lost = false;
+            uint32_t kept = 0;  // words of which this lane's id was kept
+            const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+            for (int w = 0; w < DEGW; ++w) {
+                const uint32_t k = vis.key(v[w]);
+                uint16_t* const sl = vis.slot(k);
+                const uint16_t tag = vis.tag(k);
+                bool keep = *sl != tag;
+                if (!a.distinct) {
+                    const unsigned mm = __match_any_sync(kFull, v[w]);  // all lanes
+                    keep = keep && (mm & lt) == 0;
+                    if (DEGW > 1 && w > 0 && lost && keep)
+                        for (uint32_t j = 0; j < ncand; ++j)
+                            if (cid[j] == v[w]) {
+                                keep = false;
+                                break;
+                            }
+                }
+                const unsigned kb = __ballot_sync(kFull, keep);
+                if (keep) {
+                    const uint32_t at = ncand + __popc(kb & lt);
+                    *sl = tag;
+                    cid[at] = v[w];
+                    cd[at] = sv[w];
+                }
+                ncand += __popc(kb);
+                __syncwarp();
+                if (DEGW > 1 && w + 1 < DEGW && !a.distinct) {
+                    kept |= keep ? 1u << w : 0u;
+                    bool gone = false;
+#pragma unroll
+                    for (int e = 0; e <= w; ++e) {
+                        const uint32_t ke = vis.key(v[e]);
+                        gone |= ((kept >> e) & 1u) && *vis.slot(ke) != vis.tag(ke);
+                    }
+                    lost = lost || __any_sync(kFull, gone);
+                }
+            }
+            // once rp is full, the slots' sums bound the distances
+            const bool filter = acc_n >= ef && a.esum;
+
+            if constexpr (H > 0) {
+                // the next pop is the first unpopped pool entry or an accepted
+                // candidate of this expansion: ask L2 for the pool entry's list
+                // while the distances are computed
+                if (cur < alen && lane == 0)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.nbrs + (size_t)(ai[cur] & ~kPopped) *
+                                                                         a.deg));
+            }
+            if (lane == 0) ws->calcs = ws->calcs + ncand;
+            // candidates that certainly fail the bound are not evaluated
+            if (filter && ncand > 0) {
+                const Sq8Filter f{ws->K, ws->st, ws->E};
+                ncand = filter_candidates<WIDE>(a, f, lower, planes, cid, cd, ncand, lane);
+            }
         }
 
+        qi = ws->qi;
         // Output (qg.hpp:340-343). rp pops come out in descending distance;
         // only equal distances make the heap layout decide. So when the
         // sorted pool holds exactly rp (no ties beyond the ef-th entry) and
@@ -558,10 +699,10 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
             }
         }
         if (!fail && !direct && !ra.replay_all &&
-            batch_replays_in_place(vbits, ra.scap, acap, ra.rcap)) {
+            batch_replays_in_place(32 * DEGW, vbits, ra.scap, acap, ra.rcap)) {
             __syncwarp();
-            const HeapView rph{reinterpret_cast<uint2*>(vis), nullptr, ra.rcap};
-            fail = !replay_result(a, ra, qi, acc_n, rph, lane);
+            const HeapView rph{reinterpret_cast<uint2*>(wb + L.vis), nullptr, ra.rcap};
+            fail = !replay_result_call(a, ra, qi, acc_n, rph, lane);
             direct = !fail;
         }
         if (lane == 0) {
@@ -572,7 +713,7 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
             }
             if (a.stats) {
                 *reinterpret_cast<uint4*>(a.stats + 4 * (size_t)qi) =
-                    make_uint4(pops, calcs, 0u, P);
+                    make_uint4(ws->pops, ws->calcs, 0u, P);
             }
         }
         __syncwarp();
@@ -584,14 +725,15 @@ __global__ void __launch_bounds__(H ? 32 * (H + 1) : 160, 4)
     }
 }
 
-template <int G, int DEGW, int LW, int H = 0>
-static cudaError_t batch_run(const SearchArgs& a, const ReplayArgs& ra, int warps, int blocks,
-                            cudaStream_t st, int* occ) {
+template <int DEGW, bool WIDE, int H>
+cudaError_t batch_launch_as(const SearchArgs& a, const ReplayArgs& ra, int warps, int blocks,
+                      cudaStream_t st, int* occ) {
     const size_t dpad = (a.dim + 15u) & ~15u;
     const int areas = H ? 1 : warps;
     const int threads = H ? 32 * (H + 1) : warps * 32;
-    const size_t smem = 8 * dpad + (size_t)areas * batch_warp_bytes(a.dim, a.vbits, ra.scap, ra.acap);
-    auto k = batch_search_kernel<G, DEGW, LW, H>;
+    const size_t smem =
+        8 * dpad + (size_t)areas * batch_layout(a.dim, 32 * DEGW, a.vbits, ra.scap, ra.acap).total;
+    auto k = batch_search_kernel<DEGW, WIDE, H>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, smem);
@@ -599,33 +741,11 @@ static cudaError_t batch_run(const SearchArgs& a, const ReplayArgs& ra, int warp
     return cudaGetLastError();
 }
 
-// The query-per-block form: 4 lanes per candidate, 4 warps (8 candidates
-// each); a lane holds one code word per 16-dimension chunk, so 16 words in
-// flight cover 8 chunks per round.
-template <int DEGW>
-cudaError_t batch_cta_run(const SearchArgs& a, const ReplayArgs& ra, int blocks, cudaStream_t st,
-                          int* occ) {
-    return batch_run<4, DEGW, 16, 3>(a, ra, 1, blocks, st, occ);
-}
-
-// All instances for one lanes-per-candidate G: degree words 1-4, each with
-// the short and the long code-load window.
-template <int G>
-cudaError_t batch_dispatch(const SearchArgs& a, const ReplayArgs& ra, int degw, int warps,
-                           int blocks, cudaStream_t st, int* occ) {
-    const bool wide = a.dim >= kBatchWideDim;
-#define LQG_BCASE(DW)                                                                   \
-    case DW:                                                                            \
-        return wide ? batch_run<G, DW, 32>(a, ra, warps, blocks, st, occ)               \
-                    : batch_run<G, DW, batch_load_words(DW)>(a, ra, warps, blocks, st, occ);
-    switch (degw) {
-        LQG_BCASE(1)
-        LQG_BCASE(2)
-        LQG_BCASE(3)
-        LQG_BCASE(4)
-        default: return cudaErrorInvalidValue;
-    }
-#undef LQG_BCASE
+template <int DEGW, int H = 0>
+cudaError_t batch_run(const SearchArgs& a, const ReplayArgs& ra, int warps, int blocks,
+                      cudaStream_t st, int* occ) {
+    return a.dim >= kWideDim ? batch_launch_as<DEGW, true, H>(a, ra, warps, blocks, st, occ)
+                             : batch_launch_as<DEGW, false, H>(a, ra, warps, blocks, st, occ);
 }
 
 }  // namespace lqg

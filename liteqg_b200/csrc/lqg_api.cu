@@ -77,6 +77,11 @@ lqg_status upload(lqg_index* ix) {
                           cudaMemcpyHostToDevice));
     LQG_CUDA(cudaMemcpy(ix->d_params, ix->params.data(), ix->dim * 2 * sizeof(float),
                         cudaMemcpyHostToDevice));
+    filter_alloc(ix);
+    lqg_status s;
+    if ((s = filter_node_sums(ix, nullptr)) != LQG_OK) return s;
+    if ((s = filter_edge_sums(ix, nullptr)) != LQG_OK) return s;
+    if ((s = check_distinct(ix, nullptr)) != LQG_OK) return s;
     ix->has_data = true;
     return LQG_OK;
 }
@@ -158,6 +163,8 @@ SearchArgs base_args(const lqg_index* ix, const Workspace& w, const BatchSpec& b
     a.nbrs = ix->d_nbrs;
     a.codes = ix->d_codes;
     a.params = ix->d_params;
+    a.esum = ix->d_esum;
+    a.distinct = ix->distinct;
     a.n = (uint32_t)ix->n;
     a.dim = ix->dim;
     a.deg = ix->deg;
@@ -183,6 +190,26 @@ lqg_status reset_ctl(Workspace& w, cudaStream_t st) {
     LQG_CUDA(cudaMemsetAsync(w.d_ctl, 0, kCtlWords * sizeof(uint32_t), st));
     LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlErrQuery, 0xFF, sizeof(uint32_t), st));
     return LQG_OK;
+}
+
+// Visited-cache bits of a batch-kernel launch of m queries, `warps` per block.
+// A larger cache forgets fewer nodes (at ef 200 and degree 96: 10.5 k
+// evaluations per query at 10 bits, 6.5 k at 13, 5.6 k without forgetting), but
+// costs resident queries: a batch that fills the GPU runs at the tuned 10 bits
+// (1M x 128, 10,000 queries at ef 64: 2.75 ms at 10, 2.95 at 11, 4.45 at 12).
+// So a batch whose queries all fit at once takes the largest cache they fit
+// with, when the tuning field is at its default; other values are taken as they
+// are. Ids of the index must name slot and tag uniquely (batch_kernel.cuh).
+uint32_t batch_visited_bits(const lqg_index* ix, const lqg::ReplayArgs& ra, int64_t m, int warps) {
+    uint32_t vb = ix->tune.visited_bits;
+    while (vb < 15 && ix->n > (1ull << (vb + 16))) ++vb;
+    if (vb != 10) return vb;
+    for (uint32_t x = 13; x > vb; --x) {
+        const size_t smem = lqg::batch_smem_bytes(ix->dim, ix->deg, x, ra.scap, ra.acap, warps);
+        const int64_t per_sm = std::min<int64_t>(228 * 1024 / (smem + 1024), 20 / warps);
+        if (smem <= 227 * 1024 && per_sm * warps * ix->num_sms >= m) return x;
+    }
+    return vb;
 }
 
 // Fast kernel over all queries, then the exact kernel over the flagged ones.
@@ -236,7 +263,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         int sw = plain ? 1 : (int)(split ? std::min(t.heap_warps, 5u) : t.replay_warps);
         if (batch) {
             while (sw > 1 &&
-                   lqg::batch_smem_bytes(ix->dim, t.visited_bits, ra.scap, ra.acap, sw) > 227 * 1024)
+                   lqg::batch_smem_bytes(ix->dim, ix->deg, t.visited_bits, ra.scap, ra.acap, sw) > 227 * 1024)
                 --sw;
         } else if (split) {
             while (sw > 1 && lqg::split_smem_bytes(ix->dim, t.visited_bits, ra.scap, sw) > 227 * 1024)
@@ -248,12 +275,12 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         ra.swarps = (uint32_t)sw;
         SearchArgs h = base_args(ix, w, b);
         h.qhead = w.d_ctl + kCtlHeapHead;
-        h.vbits = t.visited_bits;
+        h.vbits = batch ? batch_visited_bits(ix, ra, b.m, sw) : t.visited_bits;
         // small batches: one query per block of 4 warps, when every query of
         // the batch can be resident at once
         bool cta = false;
         if (batch && b.small_ok && t.small_batch != LQG_SMALL_BATCH_OFF &&
-            lqg::batch_smem_bytes(ix->dim, t.visited_bits, ra.scap, ra.acap, 1) <= 227 * 1024) {
+            lqg::batch_smem_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap, 1) <= 227 * 1024) {
             if (plain) {
                 cta = true;  // one query: no occupancy question
             } else {
@@ -267,10 +294,14 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
             }
         }
         if (cta) sw = 1;
+        // the batch kernels' distance passes use 4 lanes per candidate; the
+        // tuning field keeps its accepted values
+        if (batch && !cta && t.lanes_per_cand != 2 && t.lanes_per_cand != 4 && t.lanes_per_cand != 8)
+            return fail(LQG_ERR_ARG, "search kernel cannot launch with this tuning");
         auto launch = [&](const SearchArgs& c, int blocks, int* occ) {
             if (cta) return lqg::launch_batch_cta(c, ra, degw, blocks, b.st, occ);
             if (batch)
-                return lqg::launch_batch(c, ra, (int)t.lanes_per_cand, degw, sw, blocks, b.st, occ);
+                return lqg::launch_batch(c, ra, degw, sw, blocks, b.st, occ);
             return split ? lqg::launch_split(c, ra, RE, (int)t.lanes_per_cand, degw, sw, blocks, b.st, occ)
                          : lqg::launch_replay(c, ra, RE, (int)t.lanes_per_cand, degw, blocks, b.st, occ);
         };
@@ -325,7 +356,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
             e = launch(c, cb, nullptr);
             if (e != cudaSuccess) return cuda_fail(e, "search launch");
             const bool in_place =
-                batch ? lqg::batch_replays_in_place_host(t.visited_bits, ra.scap, ra.acap, ra.rcap)
+                batch ? lqg::batch_replays_in_place_host(ix->deg, h.vbits, ra.scap, ra.acap, ra.rcap)
                       : lqg::split_replays_in_place_host(t.visited_bits, ra.scap, ra.rcap);
             if (!split || ra.replay_all || !in_place) {
                 e = lqg::launch_rp_replay(c, ra, b.st);
@@ -817,7 +848,7 @@ lqg_status lqg_set_tuning(lqg_index* ix, const lqg_tuning* t) {
         return fail(LQG_ERR_ARG, "replay kernel tuning needs more than 227 KB of shared memory");
     if (n.mode == 4 && lqg::split_smem_bytes(ix->dim, n.visited_bits, n.heap_scap, 1) > 227 * 1024)
         return fail(LQG_ERR_ARG, "split kernel tuning needs more than 227 KB of shared memory");
-    if (n.mode >= 5 && lqg::batch_smem_bytes(ix->dim, n.visited_bits, n.heap_scap,
+    if (n.mode >= 5 && lqg::batch_smem_bytes(ix->dim, ix->deg, n.visited_bits, n.heap_scap,
                                              32u * (uint32_t)lqg::replay_pool_regs(kMaxEf), 1) >
                            227 * 1024)
         return fail(LQG_ERR_ARG, "batch kernel tuning needs more than 227 KB of shared memory");
@@ -907,6 +938,9 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
     dfree(ix->d_nbrs);
     dfree(ix->d_codes);
     dfree(ix->d_params);
+    dfree(ix->d_nsum);
+    dfree(ix->d_esum);
+    ix->distinct = 0;
 
     const uint32_t rest_stride = 64, rev_cap = deg;
     const uint64_t chunk = std::min<uint64_t>(n, 1u << 20);
@@ -1079,6 +1113,12 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
         LQG_BCUDA(timed_prune(b, n), "merge reverse edges");
         LQG_BCUDA(lqg::launch_random_fill(d_new, d_new_cnt, n, deg, seed + 1 + it, st), "fill");
         LQG_BCUDA(cudaMemcpy(ix->d_nbrs, d_new, n * deg * 4, cudaMemcpyDeviceToDevice), "graph");
+    }
+    filter_alloc(ix);
+    if ((s = filter_node_sums(ix, st)) != LQG_OK || (s = filter_edge_sums(ix, st)) != LQG_OK ||
+        (s = check_distinct(ix, st)) != LQG_OK) {
+        cleanup();
+        return s;
     }
     LQG_BCUDA(cudaMemcpy(ix->nbrs.data(), ix->d_nbrs, n * deg * 4, cudaMemcpyDeviceToHost), "graph");
     LQG_BCUDA(cudaMemcpy2D(ix->codes.data(), dim, ix->d_codes, ix->cstride, dim, n,

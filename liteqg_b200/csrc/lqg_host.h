@@ -209,6 +209,11 @@ struct lqg_index {
     uint32_t* d_nbrs = nullptr;
     uint8_t* d_codes = nullptr;
     float* d_params = nullptr;
+    // sums of the integer distance bound (filter.cu); NULL when they did not
+    // fit in device memory (the kernels then evaluate every candidate)
+    float* d_nsum = nullptr;  // [n]
+    float* d_esum = nullptr;  // [n][deg]
+    uint32_t distinct = 0;    // no neighbour list holds an id twice
 
     lqg_host::Workspace ws;  // the default work area (one batch at a time)
     lqg_host::FsSection fs;  // FastScan section (empty until built or loaded)
@@ -226,6 +231,8 @@ struct lqg_index {
         lqg_host::dfree(d_nbrs);
         lqg_host::dfree(d_codes);
         lqg_host::dfree(d_params);
+        lqg_host::dfree(d_nsum);
+        lqg_host::dfree(d_esum);
         ws.release();
         fs.release();
         if (own_stream) cudaStreamDestroy(own_stream);
@@ -236,6 +243,13 @@ struct lqg_index {
 namespace lqg_host {
 lqg_status check_batch(lqg_index* ix, BatchSpec& b);
 lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain);
+// Sums of the integer distance bound (filter.cu): buffers, per-node sums of
+// the current codes, per-slot sums of the current lists.
+void filter_alloc(lqg_index* ix);
+// Whether any list of the index holds an id twice (sets ix->distinct; waits).
+lqg_status check_distinct(lqg_index* ix, cudaStream_t st);
+lqg_status filter_node_sums(lqg_index* ix, cudaStream_t st);
+lqg_status filter_edge_sums(lqg_index* ix, cudaStream_t st);
 // Work order of a batch (order.cu): largest ef, then farthest from the entry
 // point, first.
 lqg_status ensure_order(Workspace& w, int64_t chunk);

@@ -29,6 +29,8 @@ struct SearchArgs {
     const uint32_t* nbrs;    // [n][deg]
     const uint8_t* codes;    // [n][cstride]
     const float* params;     // [dim][2] (min, scale)
+    const float* esum;       // [n][deg] sums of the distance bound (sq8_filter.cuh), or NULL
+    uint32_t distinct;       // no neighbour list holds an id twice
     uint32_t n, dim, deg, cstride, entry;
     const float* queries;    // [m][dim]
     int64_t m;               // number of queries in the work list

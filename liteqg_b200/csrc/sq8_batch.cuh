@@ -55,6 +55,7 @@ __device__ __forceinline__ void eval_batch(const SearchArgs& a, const uint32_t* 
 #pragma unroll
         for (int t = 0; t < AP; ++t) acc2[p][t] = 0ull;
     }
+#pragma unroll 1
     for (uint32_t b0 = 0; b0 < mul; b0 += 16 * U) {
         if constexpr (PF != 0) {
 #pragma unroll
@@ -169,6 +170,129 @@ __device__ __forceinline__ void eval_batch(const SearchArgs& a, const uint32_t* 
             cd[c] = res;
         }
     }
+}
+
+// The same distances for few candidates: 8 lanes per candidate (2 dimensions
+// of every 16-byte chunk each), candidates cid[base, base + 4 NP) per call; NP
+// rows per lane share the query, minimum and scale loads. Groups past the last
+// candidate repeat it (no predicates on the loads). A row goes in blocks of 4
+// chunks with no branch inside, so that the loads of a block and the
+// arithmetic of its chunks overlap.
+template <int NP>
+__device__ __forceinline__ void eval_few(const SearchArgs& a, const uint32_t* cid, float* cd,
+                                         uint32_t base, uint32_t ncand, const float* __restrict__ qs,
+                                         const float* __restrict__ pmin,
+                                         const float* __restrict__ pscale, int lane) {
+    const int g = lane >> 3, r = lane & 7;
+    const uint32_t dim = a.dim;
+    const uint32_t mul = dim & ~15u;
+    const unsigned long long C23 = pk(0x4B000000u, 0x4B000000u);
+    const uint8_t* p[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i)
+        p[i] = a.codes + (size_t)cid[min(base + 4 * i + g, ncand - 1)] * a.cstride + 2 * r;
+    const float* ql = qs + 2 * r;
+    const float* ml = pmin + 2 * r;
+    const float* sl = pscale + 2 * r;
+    unsigned long long acc[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) acc[i] = 0ull;
+    auto load = [&](int i, uint32_t d) -> uint32_t {
+        return __ldg(reinterpret_cast<const unsigned short*>(p[i] + d));
+    };
+    // t = q - dec of this lane's 2 dimensions of the chunk at d, for every row
+    auto diff = [&](const uint32_t (&w)[NP], uint32_t d, unsigned long long (&t)[NP]) {
+        const unsigned long long q = *reinterpret_cast<const unsigned long long*>(ql + d);
+        const unsigned long long m = *reinterpret_cast<const unsigned long long*>(ml + d);
+        const unsigned long long s = *reinterpret_cast<const unsigned long long*>(sl + d);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            const unsigned long long c = sub2(pk(__byte_perm(w[i], 0x4B000000u, 0x7440u),
+                                                 __byte_perm(w[i], 0x4B000000u, 0x7441u)), C23);
+            t[i] = sub2(q, fma2(c, s, m));
+        }
+    };
+    uint32_t b = 0;
+    if (mul >= 64) {
+        uint32_t w[4][NP];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int i = 0; i < NP; ++i) w[u][i] = load(i, 16 * u);
+#pragma unroll 1
+        for (; b + 64 <= mul; b += 64) {
+            uint32_t n[4][NP];
+            const uint32_t nb = min(b + 64, mul - 64);  // the next block (the last one again)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int i = 0; i < NP; ++i) n[u][i] = load(i, nb + 16 * u);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                unsigned long long t[NP];
+                diff(w[u], b + 16 * u, t);
+#pragma unroll
+                for (int i = 0; i < NP; ++i) acc[i] = fma2(t[i], t[i], acc[i]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int i = 0; i < NP; ++i) w[u][i] = n[u][i];
+        }
+    }
+#pragma unroll 1
+    for (; b < mul; b += 16) {
+        uint32_t w[NP];
+        unsigned long long t[NP];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) w[i] = load(i, b);
+        diff(w, b, t);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) acc[i] = fma2(t[i], t[i], acc[i]);
+    }
+    // the AVX-512 reduction tree (l2.hpp:16-35): fold 8, 4, 2, 1
+    float res[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        float x[2];
+        upk(acc[i], x[0], x[1]);
+#pragma unroll
+        for (int h = 4; h >= 1; h >>= 1)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) x[t] = __fadd_rn(x[t], __shfl_down_sync(kFull, x[t], h));
+        res[i] = __fadd_rn(x[0], x[1]);
+    }
+    if (mul < dim) {  // warp-uniform: the scalar tail, in increasing dimension
+        uint32_t w[NP];
+        unsigned long long t[NP];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) w[i] = load(i, mul);
+        diff(w, mul, t);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            float x[2];
+            upk(t[i], x[0], x[1]);
+#pragma unroll 1
+            for (uint32_t e = 0; mul + e < dim; ++e) {
+                const float df = __shfl_sync(kFull, e & 1 ? x[1] : x[0], (lane & ~7) + (e >> 1));
+                res[i] = __fmaf_rn(df, df, res[i]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NP; ++i)
+        if (r == 0 && base + 4 * i + g < ncand) cd[base + 4 * i + g] = res[i];
+}
+
+// Distances of cid[0, n) into cd by one warp: 8 candidates at a time, a last
+// group of up to 4 at half the work.
+__device__ __forceinline__ void eval_list(const SearchArgs& a, const uint32_t* cid, float* cd,
+                                          uint32_t n, const float* qs, const float* pmin,
+                                          const float* pscale, int lane) {
+    uint32_t b = 0;
+#pragma unroll 1
+    for (; b + 4 < n; b += 8) eval_few<2>(a, cid, cd, b, n, qs, pmin, pscale, lane);
+    if (b < n) eval_few<1>(a, cid, cd, b, n, qs, pmin, pscale, lane);
 }
 
 }  // namespace lqg

@@ -37,7 +37,7 @@
 // against rp.top() (replay_result, heap_ops.cuh).
 //
 // Visited set: a direct-mapped cache of evaluated ids in shared memory (16-bit
-// tags, VisitedCache below). It may forget an id, never invents one. A forgotten node that is evaluated
+// tags, VisitedCache in lqg_kernels.cuh). It may forget an id, never invents one. A forgotten node that is evaluated
 // again has its old distance; if it passes the bound now it was accepted
 // before and is still in the sorted pool with the same id and distance, and
 // it is dropped there.
@@ -76,24 +76,6 @@ __host__ __device__ inline BatchLayout batch_layout(uint32_t dim, uint32_t deg, 
     L.total = L.pool + 8u * acap;
     return L;
 }
-
-// The visited cache: 2^(vbits + 1) slots of 16 bits. An id's low B = vbits + 16
-// bits times an odd constant is a bijection on B bits; the top vbits + 1 bits
-// are the slot and the other 15 the tag (0x8000 set: taken), so slot and tag
-// name exactly one id as long as ids are below 2^B (the launcher sees to it).
-// Twice the slots of 32-bit ids in the same bytes: 6 % fewer evaluations at ef
-// 64, 13 % at ef 200 and degree 96.
-struct VisitedCache {
-    uint16_t* s;
-    uint32_t vbits;
-    __device__ __forceinline__ uint32_t key(uint32_t id) const {
-        return (id * 0x9E3779B1u) << (16u - vbits);  // B bits at the top
-    }
-    __device__ __forceinline__ uint16_t* slot(uint32_t k) const { return s + (k >> (31u - vbits)); }
-    __device__ __forceinline__ uint16_t tag(uint32_t k) const {
-        return (uint16_t)((k >> (16u - vbits)) | 0x8000u);
-    }
-};
 
 // Per-query values that are read once or twice per pop: kept in shared memory,
 // so that the search loop's registers hold only what every step needs.

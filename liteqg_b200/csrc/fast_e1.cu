@@ -2,6 +2,5 @@
 #include "fast_kernel.cuh"
 
 namespace lqg {
-template cudaError_t fast_dispatch<1>(const SearchArgs&, int, int, int, int, size_t,
-                                       cudaStream_t, int*);
+template cudaError_t fast_dispatch<1>(const SearchArgs&, int, int, int, size_t, cudaStream_t, int*);
 }  // namespace lqg

@@ -13,11 +13,16 @@
 //   sp but later trims from rp are then strictly above every later bound and
 //   never pop. The kernel therefore keeps only the ef-pool, sorted, in
 //   registers (E entries per lane), with the "expanded" bit in the id.
+//   Once the pool is full, the integer bound of sq8_filter.cuh drops the
+//   candidates that certainly fail it before any exact distance is computed.
 //   The visited set is a direct-mapped cache of evaluated ids in shared
-//   memory: it may forget an id but never reports an unvisited one, and a
-//   forgotten id that is evaluated again has the same distance, so it either
-//   fails the bound or meets its own pool entry (same id, same distance) and
-//   is dropped. Candidates are merged in ascending distance; any equality
+//   memory (VisitedCache): it may forget an id but never reports an unvisited
+//   one, and a forgotten id that is evaluated again has the same distance, so
+//   it either fails the bound or meets its own pool entry (same id, same
+//   distance) and is dropped. With lists of more than one 32-id word, equal
+//   distances of one expansion go by the candidates' places after the filter
+//   of a 2^vbits-slot cache of full ids (lane, then word), so that cache is
+//   kept too: it decides the places, the other one what is evaluated. Candidates are merged in ascending distance; any equality
 //   between a candidate and the pool, or between two candidates, with
 //   different ids (or a non-finite distance) hands the query to the exact
 //   kernel, since only there does the reference's heap layout decide.
@@ -34,14 +39,9 @@
 #include "lqg_internal.h"
 #include "lqg_kernels.cuh"
 #include "sq8_batch.cuh"
+#include "sq8_filter.cuh"
 
 namespace lqg {
-
-// Code words in flight per lane in the fast kernel's distance batches: the
-// 512-entry pool (E = 16) holds 32 registers per lane, so it gets the short
-// window.
-template <int E>
-constexpr int kFastLoadWords = E >= 16 ? 8 : 16;
 
 template <int E>
 __device__ __forceinline__ float pool_at(const float (&pd)[E], uint32_t lane_of, uint32_t slot_of) {
@@ -52,8 +52,18 @@ __device__ __forceinline__ float pool_at(const float (&pd)[E], uint32_t lane_of,
     return __shfl_sync(kFull, v, lane_of);
 }
 
-template <int E, int G, int DEGW>
-__global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
+// Shared memory of one warp: the query, its byte planes, the cache of evaluated
+// nodes, the place cache (lists of several words), candidate ids, distances and
+// places.
+__host__ __device__ inline uint32_t fast_warp_bytes(uint32_t dim, uint32_t deg, uint32_t vbits,
+                                                    uint32_t sbits) {
+    return 4u * ((dim + 15u) & ~15u) + 2u * filter_plane(dim) + (4u << sbits) +
+           (deg > 32 ? 4u << vbits : 0u) + 12u * deg;
+}
+
+template <int E, int DEGW>
+__global__ void __launch_bounds__(512)
+    fast_search_kernel(const __grid_constant__ SearchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -62,12 +72,15 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
     float* pmin = reinterpret_cast<float*>(smem);
     float* pscale = pmin + dpad;
     const uint32_t vbits = a.vbits;
-    const uint32_t vsize = 1u << vbits;
-    unsigned char* wb = smem + 8u * dpad + (size_t)warp * (4u * dpad + 4u * vsize + kCandBytes);
+    unsigned char* wb = smem + 8u * dpad + warp * fast_warp_bytes(dim, 32 * DEGW, vbits, a.sbits);
     float* qs = reinterpret_cast<float*>(wb);
-    uint32_t* vis = reinterpret_cast<uint32_t*>(wb + 4u * dpad);
-    uint32_t* cid = vis + vsize;
-    float* cd = reinterpret_cast<float*>(cid + kMaxDeg);
+    int8_t* planes = reinterpret_cast<int8_t*>(wb + 4u * dpad);
+    unsigned char* vb = wb + 4u * dpad + 2u * filter_plane(dim);
+    const VisitedCache vis{reinterpret_cast<uint16_t*>(vb), a.sbits};
+    uint32_t* place = reinterpret_cast<uint32_t*>(vb + (4u << a.sbits));  // DEGW > 1
+    uint32_t* cid = place + (DEGW > 1 ? 1u << vbits : 0u);
+    float* cd = reinterpret_cast<float*>(cid + 32 * DEGW);
+    uint32_t* cpl = reinterpret_cast<uint32_t*>(cd + 32 * DEGW);  // places (DEGW > 1)
 
     for (uint32_t i = threadIdx.x; i < dpad; i += blockDim.x) {
         pmin[i] = i < dim ? a.params[2 * i] : 0.f;
@@ -75,9 +88,9 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
     }
     __syncthreads();
 
-    const int g = lane / G, r = lane % G;
-    constexpr int CPP = 32 / G;
     const uint32_t lt = lanemask_lt();
+    float smax, n2;
+    filter_index_sums(pmin, pscale, dim, lane, smax, n2);
     const int64_t mlist = a.nlist ? (int64_t)*a.nlist : a.m;
     const float INF = CUDART_INF_F;
 
@@ -91,9 +104,18 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
         ef = min(max(ef, 1u), 32u * E);
         const uint32_t k = min(a.kq ? a.kq[qi] : a.k0, a.kstride);
         const float* q = a.queries + (size_t)qi * dim;
+#pragma unroll 1
         for (uint32_t i = lane; i < dpad; i += 32) qs[i] = i < dim ? q[i] : 0.f;
-        for (uint32_t i = lane; i < vsize; i += 32) vis[i] = kNoId;
+#pragma unroll 1
+        for (uint32_t i = 4 * lane; i < (1u << a.sbits); i += 128)
+            *reinterpret_cast<uint4*>(vis.s + 2 * i) = make_uint4(0, 0, 0, 0);
+        if (DEGW > 1)
+#pragma unroll 1
+            for (uint32_t i = 4 * lane; i < (1u << vbits); i += 128)
+                *reinterpret_cast<uint4*>(place + i) = make_uint4(kNoId, kNoId, kNoId, kNoId);
+        if (lane == 0) cid[0] = a.entry;
         __syncwarp();
+        const Sq8Filter flt = filter_prepare(qs, pmin, pscale, dim, smax, n2, planes, lane);
 
         float pd[E];
         uint32_t pi[E];
@@ -105,14 +127,16 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
 
         // qg.hpp:305-311: the entry point seeds both pools and is visited.
         const uint32_t ep = a.entry;
-        float d0 = sq8_l2_group<G>(a.codes + (size_t)ep * a.cstride, g == 0, qs, pmin,
-                                   pscale, dim, r);
-        d0 = __shfl_sync(kFull, d0, 0);
+        eval_list(a, cid, cd, 1, qs, pmin, pscale, lane);
+        __syncwarp();
+        const float d0 = cd[0];
         bool tie = !(d0 < INF) && !a.ties_ok;
         if (lane == 0) {
             pd[0] = d0;
             pi[0] = ep;
-            vis[hash_id(ep, vbits)] = ep;
+            const uint32_t k = vis.key(ep);
+            *vis.slot(k) = vis.tag(k);
+            if (DEGW > 1) place[hash_id(ep, vbits)] = ep;
         }
         __syncwarp();
         uint32_t pops = 0, calcs = 1;
@@ -146,53 +170,59 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
             // qg.hpp:320-324: neighbours in list order, unvisited ones kept.
             uint32_t ncand = 0;
             const uint32_t* nb = a.nbrs + (size_t)u * a.deg;
+            const float T0 = pool_at<E>(pd, tl, ts);  // +inf until the pool is full
+            const bool filter = T0 < INF && a.esum;
             uint32_t v[DEGW];
+            float sv[DEGW];
 #pragma unroll
             for (int w = 0; w < DEGW; ++w) v[w] = __ldg(nb + w * 32 + lane);
 #pragma unroll
+            for (int w = 0; w < DEGW; ++w)
+                sv[w] = filter ? __ldg(a.esum + (size_t)u * a.deg + w * 32 + lane) : 0.f;
+            uint32_t nplace = 0;
+#pragma unroll
             for (int w = 0; w < DEGW; ++w) {
+                const uint32_t k = vis.key(v[w]);
+                uint16_t* const sl = vis.slot(k);
+                const uint16_t tag = vis.tag(k);
+                bool keep = *sl != tag;
+                bool placed = true;
                 const uint32_t h = hash_id(v[w], vbits);
-                const bool seen = vis[h] == v[w];
-                const unsigned mm = __match_any_sync(kFull, v[w]);
-                const bool keep = !seen && (mm & lt) == 0;
-                __syncwarp();
-                if (keep) vis[h] = v[w];
+                if (DEGW > 1) placed = place[h] != v[w];
+                if (!a.distinct) {
+                    const unsigned mm = __match_any_sync(kFull, v[w]);  // all lanes
+                    const bool first = (mm & lt) == 0;
+                    keep = keep && first;
+                    placed = placed && first;
+                }
+                if (DEGW > 1) keep = keep && placed;  // an evaluated node may be forgotten here only
                 const unsigned kb = __ballot_sync(kFull, keep);
-                if (keep) cid[ncand + __popc(kb & lt)] = v[w];
+                const unsigned pb = DEGW > 1 ? __ballot_sync(kFull, placed) : 0u;
+                if (keep) {
+                    const uint32_t at = ncand + __popc(kb & lt);
+                    *sl = tag;
+                    cid[at] = v[w];
+                    cd[at] = sv[w];
+                    if (DEGW > 1) cpl[at] = nplace + __popc(pb & lt);
+                }
+                if (DEGW > 1 && placed) place[h] = v[w];
                 ncand += __popc(kb);
+                nplace += __popc(pb);
                 __syncwarp();
             }
 
-            // qg.hpp:325-328: SQ8 decode + L2 of every kept neighbour. Rows
-            // below 256 bytes with up to 4 lanes per candidate: the packed-pair
-            // batch routine (32 candidates per call, code loads of every pass
-            // issued before the arithmetic; the same operations in the same
-            // order). Longer rows, or wider groups: one candidate per group at
-            // a time with 8 chunks of the row in flight (the batch routine's
-            // short load window would take a dependent round per two chunks).
-            bool packed = false;
-            if constexpr (G <= 4) packed = dim < kBatchWideDim;
-            if (packed) {
-                if constexpr (G <= 4)
-                    for (uint32_t b = 0; b < ncand; b += 32)
-                        eval_batch<G, G, kFastLoadWords<E>, 1>(a, cid, cd, b, ncand, qs, pmin,
-                                                               pscale, g, r);
-            } else {
-                for (uint32_t base = 0; base < ncand; base += CPP) {
-                    const uint32_t c = base + g;
-                    const bool valid = c < ncand;
-                    const uint32_t id = valid ? cid[c] : 0u;
-                    const float d = sq8_l2_group<G>(a.codes + (size_t)id * a.cstride, valid, qs,
-                                                    pmin, pscale, dim, r);
-                    if (valid && r == 0) cd[c] = d;
-                }
-            }
-            calcs += ncand;
+            // qg.hpp:325-328: SQ8 decode + L2 of the kept neighbours that may
+            // still pass the bound
+            calcs += DEGW > 1 ? nplace : ncand;
+            if (filter && ncand > 0)
+                ncand = filter_candidates<true, (DEGW > 1)>(a, flt, T0, planes, cid, cd, ncand, lane,
+                                                            cpl);
+            eval_list(a, cid, cd, ncand, qs, pmin, pscale, lane);
             __syncwarp();
 
             // qg.hpp:329-335: pool <- ef smallest of (pool + candidates).
-            float T = pool_at<E>(pd, tl, ts);
-            uint32_t key[DEGW], cv[DEGW];
+            float T = T0;
+            uint32_t key[DEGW], cv[DEGW], ord[DEGW];
             bool bad = false;
 #pragma unroll
             for (int w = 0; w < DEGW; ++w) {
@@ -200,6 +230,9 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
                 const bool valid = c < ncand;
                 const float dc = valid ? cd[c] : INF;
                 cv[w] = valid ? cid[c] : 0u;
+                // equal distances: by place, lane first, then word
+                const uint32_t pl = DEGW > 1 && valid ? cpl[c] : 0u;
+                ord[w] = DEGW > 1 ? ((pl & 31u) << 8) | (pl >> 5) : 0u;
                 bad |= valid && !(dc < INF);
                 key[w] = (valid && dc < T) ? __float_as_uint(dc) : 0xFFFFFFFFu;
             }
@@ -213,16 +246,20 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
                 for (int w = 1; w < DEGW; ++w) lk = min(lk, key[w]);
                 const uint32_t mn = __reduce_min_sync(kFull, lk);
                 if (mn == 0xFFFFFFFFu) break;
-                int src_w = DEGW - 1;
+                // this lane's first holder of the smallest distance
+                uint32_t mine = cv[0], lo = 0xFFFFFFFFu;
 #pragma unroll
-                for (int w = DEGW - 1; w >= 0; --w)
-                    if (key[w] == mn) src_w = w;
-                const unsigned hold = __ballot_sync(kFull, lk == mn);
+                for (int w = 0; w < DEGW; ++w)
+                    if (key[w] == mn && (DEGW == 1 || ord[w] < lo)) {
+                        lo = ord[w];
+                        mine = cv[w];
+                    }
+                unsigned hold = __ballot_sync(kFull, lk == mn);
+                if (DEGW > 1 && (hold & (hold - 1u))) {
+                    const uint32_t first = __reduce_min_sync(kFull, lo);
+                    hold = __ballot_sync(kFull, lo == first);
+                }
                 const int src = __ffs(hold) - 1;
-                uint32_t mine = cv[0];
-#pragma unroll
-                for (int w = 1; w < DEGW; ++w)
-                    if (src_w == w) mine = cv[w];
                 const uint32_t cidv = __shfl_sync(kFull, mine, src);
                 // holders of the same id are one node: drop them; a holder
                 // with another id is a tie (left in place for ties_ok)
@@ -330,50 +367,30 @@ __global__ void __launch_bounds__(512) fast_search_kernel(SearchArgs a) {
     }
 }
 
-template <int E, int G, int DEGW>
+// Launches the instance, or, with occ != null, reports its resident blocks per
+// SM (0 if it cannot launch).
+template <int E, int DEGW>
 static cudaError_t run_fast(const SearchArgs& a, int warps, int blocks, size_t smem,
-                            cudaStream_t st) {
-    auto k = fast_search_kernel<E, G, DEGW>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                            cudaStream_t st, int* occ) {
+    auto k = fast_search_kernel<E, DEGW>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
+    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, warps * 32, smem);
     k<<<blocks, warps * 32, smem, st>>>(a);
     return cudaGetLastError();
 }
 
-template <int E, int G, int DEGW>
-static int occ_of(int warps, size_t smem) {
-    auto k = fast_search_kernel<E, G, DEGW>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return 0;
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, warps * 32, smem) != cudaSuccess)
-        return 0;
-    return nb;
-}
-
-// All instances for one pool size E: lanes per candidate G x degree words.
+// All instances for one pool size E: an instance per degree word count.
 template <int E>
-cudaError_t fast_dispatch(const SearchArgs& a, int G, int degw, int warps, int blocks,
-                          size_t smem, cudaStream_t st, int* occ) {
-#define LQG_CASE(GG, DW)                                              \
-    if (G == GG && degw == DW) {                                      \
-        if (occ) {                                                    \
-            *occ = occ_of<E, GG, DW>(warps, smem);                    \
-            return cudaSuccess;                                       \
-        }                                                             \
-        return run_fast<E, GG, DW>(a, warps, blocks, smem, st);       \
+cudaError_t fast_dispatch(const SearchArgs& a, int degw, int warps, int blocks, size_t smem,
+                          cudaStream_t st, int* occ) {
+    switch (degw) {
+        case 1: return run_fast<E, 1>(a, warps, blocks, smem, st, occ);
+        case 2: return run_fast<E, 2>(a, warps, blocks, smem, st, occ);
+        case 3: return run_fast<E, 3>(a, warps, blocks, smem, st, occ);
+        case 4: return run_fast<E, 4>(a, warps, blocks, smem, st, occ);
+        default: return cudaErrorInvalidValue;
     }
-#define LQG_CASES(GG) LQG_CASE(GG, 1) LQG_CASE(GG, 2) LQG_CASE(GG, 3) LQG_CASE(GG, 4)
-    LQG_CASES(1)
-    LQG_CASES(2)
-    LQG_CASES(4)
-    LQG_CASES(8)
-    LQG_CASES(16)
-#undef LQG_CASES
-#undef LQG_CASE
-    return cudaErrorInvalidValue;
 }
 
 }  // namespace lqg

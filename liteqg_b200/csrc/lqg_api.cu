@@ -395,18 +395,31 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         a.path_stride = b.path_stride;
         a.qlist = order;
         int warps = plain ? 1 : (int)t.warps_per_block;
+        while (warps > 1 &&
+               lqg::fast_smem_bytes(ix->dim, ix->deg, a.vbits, 9, warps) > 227 * 1024)
+            --warps;
+        // The cache of evaluated nodes: the largest that costs no resident
+        // warps (each node that it forgets is bounded again, once per pop that
+        // lists it); at least what names the index's ids uniquely.
+        uint32_t smin = 9;
+        while (smin < 15 && ix->n > (1ull << (smin + 16))) ++smin;
+        a.sbits = plain ? std::max(smin, 12u) : smin;
         int blocks = 1;
         if (!plain) {
-            int occ = t.blocks_per_sm ? (int)t.blocks_per_sm
-                                      : lqg::fast_occupancy(E, (int)t.lanes_per_cand, degw, warps,
-                                                            ix->dim, t.visited_bits);
+            int occ = lqg::fast_occupancy(E, degw, warps, ix->dim, a.vbits, smin);
             if (occ <= 0) return fail(LQG_ERR_ARG, "fast kernel cannot launch with this tuning");
+            for (uint32_t x = 13; x > smin; --x)
+                if (lqg::fast_occupancy(E, degw, warps, ix->dim, a.vbits, x) >= occ) {
+                    a.sbits = x;
+                    break;
+                }
+            if (t.blocks_per_sm) occ = (int)t.blocks_per_sm;
             blocks = occ * ix->num_sms;
             const int64_t need = (b.m + warps - 1) / warps;
             if (need < blocks) blocks = (int)need;
         }
         if (ix->ev_start) LQG_CUDA(cudaEventRecord(ix->ev_start, b.st));
-        e = lqg::launch_fast(a, E, (int)t.lanes_per_cand, degw, warps, blocks, b.st);
+        e = lqg::launch_fast(a, E, degw, warps, blocks, b.st);
         if (e != cudaSuccess) return cuda_fail(e, "fast search launch");
     }
 
@@ -856,8 +869,11 @@ lqg_status lqg_set_tuning(lqg_index* ix, const lqg_tuning* t) {
         lqg::heap_smem_bytes(ix->dim, n.visited_bits, kMaxEf + 2, n.heap_scap, (int)n.heap_warps) >
         227 * 1024)
         return fail(LQG_ERR_ARG, "heap kernel tuning needs more than 227 KB of shared memory");
-    if (n.mode == 1 &&
-        lqg::fast_smem_bytes(ix->dim, n.visited_bits, (int)n.warps_per_block) > 227 * 1024)
+    // (a block that needs more than the query, 2^vbits ids and 1 KB per warp
+    // runs with fewer warps)
+    const size_t dpad = (ix->dim + 15u) & ~15u;
+    if (n.mode == 1 && 8 * dpad + n.warps_per_block * (4 * dpad + ((size_t)4 << n.visited_bits) + 1024) >
+                           227 * 1024)
         return fail(LQG_ERR_ARG, "tuning needs more than 227 KB of shared memory per block");
     ix->tune = n;
     return LQG_OK;
@@ -1041,10 +1057,19 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
     LQG_BCUDA(cudaMemcpy(&best, d_best, 8, cudaMemcpyDeviceToHost), "entry point");
     ix->entry = (uint32_t)(best & 0xFFFFFFFFull);
     LQG_BCUDA(lqg::launch_random_fill(ix->d_nbrs, nullptr, n, deg, seed, st), "random graph");
+    filter_alloc(ix);
+    if ((s = filter_node_sums(ix, st)) != LQG_OK) {
+        cleanup();
+        return s;
+    }
     ix->has_data = true;
     ix->fs.release();  // a new graph: any FastScan section is stale
 
     for (uint32_t it = 0; it < num_iter; ++it) {
+        if ((s = filter_edge_sums(ix, st)) != LQG_OK || (s = check_distinct(ix, st)) != LQG_OK) {
+            cleanup();
+            return s;
+        }
         for (uint64_t c0 = 0; c0 < n; c0 += chunk) {
             const uint64_t m = std::min(chunk, n - c0);
             BatchSpec b{d_x + c0 * dim, (int64_t)m, nullptr, 1, nullptr, ef_build, d_k1, 1,
@@ -1114,9 +1139,7 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
         LQG_BCUDA(lqg::launch_random_fill(d_new, d_new_cnt, n, deg, seed + 1 + it, st), "fill");
         LQG_BCUDA(cudaMemcpy(ix->d_nbrs, d_new, n * deg * 4, cudaMemcpyDeviceToDevice), "graph");
     }
-    filter_alloc(ix);
-    if ((s = filter_node_sums(ix, st)) != LQG_OK || (s = filter_edge_sums(ix, st)) != LQG_OK ||
-        (s = check_distinct(ix, st)) != LQG_OK) {
+    if ((s = filter_edge_sums(ix, st)) != LQG_OK || (s = check_distinct(ix, st)) != LQG_OK) {
         cleanup();
         return s;
     }

@@ -146,11 +146,13 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
 // past the last candidate read the last one again (no predicates, no further
 // memory traffic). Returns how many candidates are left. ncand > 0. All lanes;
 // ends synchronised.
-template <bool WIDE>
+// TAGGED: `tag` holds a word per candidate that goes with its id.
+template <bool WIDE, bool TAGGED = false>
 __device__ __forceinline__ uint32_t filter_candidates(const SearchArgs& a, const Sq8Filter f,
                                                       float lower, const int8_t* planes,
                                                       uint32_t* cid, const float* cs,
-                                                      uint32_t ncand, int lane) {
+                                                      uint32_t ncand, int lane,
+                                                      uint32_t* tag = nullptr) {
     const int g = lane >> 2, c = lane & 3;
     const uint32_t dp = filter_plane(a.dim);
     const int8_t* pl = planes + (g & 1) * dp + 16 * c;
@@ -200,8 +202,13 @@ __device__ __forceinline__ uint32_t filter_candidates(const SearchArgs& a, const
         const bool keep = (m >> (4 * (lane & 7) + (lane >> 3))) & 1u;
         const unsigned k = __ballot_sync(kFull, keep);
         const uint32_t id = keep ? cid[b + lane] : 0u;
+        const uint32_t tg = TAGGED && keep ? tag[b + lane] : 0u;
         __syncwarp();
-        if (keep) cid[out + __popc(k & ((1u << lane) - 1u))] = id;
+        if (keep) {
+            const uint32_t at = out + __popc(k & ((1u << lane) - 1u));
+            cid[at] = id;
+            if (TAGGED) tag[at] = tg;
+        }
         out += __popc(k);
         __syncwarp();
     }

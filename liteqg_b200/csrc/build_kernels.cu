@@ -242,16 +242,24 @@ __global__ void random_fill_kernel(uint32_t* __restrict__ out, const uint32_t* _
 // ---- candidate-to-candidate distances on the tensor cores (tcgen05) -------
 //
 // The prune's P x P matrix of squared distances among a node's candidates
-// (P <= 96) as one BF16 Gram matrix per 128-dimension chunk, accumulated in
-// FP32 in tensor memory: rows are the candidates minus the node's vector
-// (so norms are on the scale of the distances), rounded to BF16 and staged in
-// shared memory in the canonical K-major layout without swizzle (8-row x
-// 16-byte core matrices; the 16 core matrices of a row group's 128 dimensions
-// are 128 bytes apart (LBO), row groups 2048 bytes apart (SBO)). One thread
-// issues tcgen05.mma.cta_group::1.kind::f16 with M = 128 (rows past P are
-// zero), N = 96, K = 16 per instruction; the result is read back with
-// tcgen05.ld (warp w owns tensor-memory lanes 32w..32w+31) and
-// d~(i, j) = n~i + n~j - 2 G(i, j) with n~ the norms of the rounded rows.
+// (P <= 96) from Gram matrices accumulated in FP32 in tensor memory: rows are
+// the candidates minus the node's vector (so norms are on the scale of the
+// distances), each value split into BF16 hi + lo (x = hi + lo + r, |r| <= 2^-16
+// |x|) and staged in shared memory 64 dimensions at a time, in the canonical
+// K-major layout without swizzle (8-row x 16-byte core matrices; the 8 core
+// matrices of a row group's 64 dimensions are 128 bytes apart (LBO), row groups
+// 1024 bytes apart (SBO)). One thread issues tcgen05.mma.cta_group::1.kind::f16
+// with M = 128 (rows past P are zero), N = 96, K = 16 per instruction, hi.hi,
+// hi.lo and lo.hi into one accumulator, so row j of it is G(j, .) complete; the
+// result is read back with tcgen05.ld (warp w owns tensor-memory lanes
+// 32w..32w+31) and d~(i, j) = n~i + n~j - 2 G(i, j) with n~ the norms in the
+// split's form. The distances never leave registers: the thread of row j takes
+// its row's decisions as the columns arrive.
+//
+// The kernel is bound by latency, so blocks per SM count: one 128-column
+// accumulator (four blocks share an SM's 512 columns) and one or two 32 KB
+// operand buffers; with two accumulators, a transposing pass through a 36 KB
+// pair buffer and 128-dimension tiles two blocks fit.
 namespace tc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -334,45 +342,54 @@ __device__ __forceinline__ void ld16(uint32_t taddr, float (&v)[16]) {
 
 // One CTA (kPruneThreads) per node.
 //  1. Gather candidates from up to three sources (pool rows, neighbour rows
-//     with counts, reverse rows with counts); drop the node and duplicates.
+//     with counts, reverse rows with counts); drop the node and, by a hash
+//     table in shared memory, duplicates.
 //  2. Exact FP32 distance node -> candidate (reference 16-lane order).
-//  3. Sort ascending (bitonic, kCandMax), keep the nearest kPruneMax.
+//  3. Sort ascending by (distance, id) (bitonic, kCandMax keys, two per thread,
+//     by shuffles), keep the nearest kPruneMax.
 //  4. Candidate-to-candidate distances, then the greedy RNG prune.
 //  5. Write up to deg kept ids; with fill, pad to exactly deg with the pruned
 //     candidates in distance order (the spirit of graph_refine,
 //     qg_builder.hpp:293-348) and mark the row count; rest rows receive the
 //     pruned candidates for a later fill.
+// Against two block-wide sorts of 36 barriers each and the two-accumulator form
+// (prune launches of a whole build, one B200): 100k x 64 degree 32 105 -> 40 ms,
+// 20k x 768 degree 64 59 -> 44 ms, 20k x 128 integers 19 -> 9.5 ms.
 // TC selects the candidate-to-candidate distance form at compile time (1:
 // BF16 Gram matrices on the tensor cores, 0: FP32 on the CUDA cores), so
 // each instance holds only its own path's registers.
+constexpr int kHashBits = 9, kHashSlots = 1 << kHashBits;  // twice kCandMax
+constexpr uint32_t kOpDims = 64;               // dimensions per operand buffer
+constexpr uint32_t kOpSbo = kOpDims / 8 * 128; // bytes between row groups
+constexpr uint32_t kOpBytes = 2 * 128 * kOpDims * 2;  // hi and lo, 128 rows of BF16
+
 template <int TC>
 __global__ void __launch_bounds__(kPruneThreads) prune_kernel(PruneArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_ids[kCandMax];
     __shared__ float s_d[kCandMax];
-    __shared__ uint32_t s_cnt;
-    __shared__ uint8_t s_keep[kPruneMax];   // 1 kept
-    // FP32 path: tile [kPruneMax+1][kTileD+1] floats; tensor-core path: the
-    // BF16 hi and lo operands, 128 rows x kTileD each; then pair
-    // [kPruneMax][kPruneMax]
+    __shared__ uint32_t s_hash[kHashSlots];      // candidate ids, open addressing
+    __shared__ uint32_t s_flag[kHashSlots / 32]; // slots whose id came from a search path
+    __shared__ unsigned long long s_x[kCandMax]; // sort keys between warps
+    __shared__ uint8_t s_keep[kPruneMax];        // 1 kept
+    // FP32 path: tile [kPruneMax+1][kTileD+1] floats, then pair
+    // [kPruneMax][kPruneMax]; tensor-core path: one or two operand buffers
     float* tile = reinterpret_cast<float*>(smem);
-    float* pair = tile + (TC ? 128 * kTileD : (kPruneMax + 1) * (kTileD + 1));
+    float* pair = tile + (kPruneMax + 1) * (kTileD + 1);
 
     const uint64_t node = blockIdx.x + a.node0;
     if (node >= a.n) return;
     const int tid = threadIdx.x;
     const uint32_t dim = a.dim;
-    if (tid == 0) s_cnt = 0;
-    for (int i = tid; i < kCandMax; i += kPruneThreads) {
-        s_ids[i] = 0xFFFFFFFFu;
-        s_d[i] = CUDART_INF_F;
-    }
+    for (int i = tid; i < kCandMax; i += kPruneThreads) s_ids[i] = 0xFFFFFFFFu;
+    for (int i = tid; i < kHashSlots; i += kPruneThreads) s_hash[i] = 0xFFFFFFFFu;
+    if (tid < kHashSlots / 32) s_flag[tid] = 0;
     __syncthreads();
 
     // 1. gather into fixed slots, source after source, up to kCandMax (so the
     // candidate set does not depend on thread timing); duplicates removed
-    // below after sorting by id. Entries are id << 1 | from_path (ids < 2^31);
-    // the node itself and out-of-range ids become empty slots.
+    // below. Entries are id << 1 | from_path (ids < 2^31); the node itself and
+    // out-of-range ids become empty slots.
     auto put = [&](uint32_t slot, uint32_t v, uint32_t from_path) {
         s_ids[slot] = (v == (uint32_t)node || v >= a.n) ? 0xFFFFFFFFu : ((v << 1) | from_path);
     };
@@ -401,60 +418,86 @@ __global__ void __launch_bounds__(kPruneThreads) prune_kernel(PruneArgs a) {
         off += c;
     }
     __syncthreads();
-    const uint32_t cnt = off;
 
-    // 2. exact distances node -> candidate (ids first sorted to drop dups)
-    // bitonic sort by id to find duplicates
-    for (uint32_t k = 2; k <= kCandMax; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = tid; i < kCandMax; i += kPruneThreads) {
-                const uint32_t l = i ^ j;
-                if (l > i) {
-                    const bool up = (i & k) == 0;
-                    const uint32_t x = s_ids[i], y = s_ids[l];
-                    if ((x > y) == up) {
-                        s_ids[i] = y;
-                        s_ids[l] = x;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
+    // 2. one copy of every id (flagged if any copy came from a search path):
+    // the first thread to enter it in the table takes it, whichever copy that
+    // is, so the set does not depend on timing. Then its exact distance from
+    // the node.
     const float* xn = a.x + node * dim;
     // rows start on 16-byte boundaries: four floats per load
     const bool v4 = (dim & 3u) == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15u) == 0;
-    for (uint32_t i = tid; i < cnt; i += kPruneThreads) {
-        const uint32_t v = s_ids[i];
-        // keep the last of equal ids (the path-flagged copy, if any)
-        const bool dup = i + 1 < cnt && (s_ids[i + 1] >> 1) == (v >> 1);
-        const float* xv = a.x + (uint64_t)(v >> 1) * dim;
-        s_d[i] = (dup || v == 0xFFFFFFFFu) ? CUDART_INF_F
-                 : v4                      ? l2_ref_order_v4(xn, xv, dim)
-                                           : l2_ref_order(xn, xv, dim);
-    }
-    __syncthreads();
-    // 3. sort ascending by (distance, id)
-    for (uint32_t k = 2; k <= kCandMax; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = tid; i < kCandMax; i += kPruneThreads) {
-                const uint32_t l = i ^ j;
-                if (l > i) {
-                    const bool up = (i & k) == 0;
-                    const float dx = s_d[i], dy = s_d[l];
-                    const uint32_t ix = s_ids[i], iy = s_ids[l];
-                    const bool gt = dx > dy || (dx == dy && ix > iy);
-                    if (gt == up) {
-                        s_d[i] = dy;
-                        s_d[l] = dx;
-                        s_ids[i] = iy;
-                        s_ids[l] = ix;
-                    }
-                }
-            }
-            __syncthreads();
+    uint32_t mine[2];  // slots of this thread's candidates in the table
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const uint32_t v = s_ids[tid + e * kPruneThreads];
+        mine[e] = 0xFFFFFFFFu;
+        if (v != 0xFFFFFFFFu) {
+            uint32_t h = ((v >> 1) * 0x9E3779B1u) >> (32 - kHashBits);
+            uint32_t was;
+            // at most kCandMax ids in twice as many slots: an end is always met
+            while ((was = atomicCAS(&s_hash[h], 0xFFFFFFFFu, v >> 1)) != 0xFFFFFFFFu && was != v >> 1)
+                h = (h + 1) & (kHashSlots - 1);
+            if (was == 0xFFFFFFFFu) mine[e] = h;
+            if (v & 1u) atomicOr(&s_flag[h >> 5], 1u << (h & 31));
         }
     }
+    __syncthreads();
+    // sort keys: distance bits (non-negative floats order as their bits), then
+    // id << 1 | flag; a slot without a candidate sorts last
+    unsigned long long key[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        key[e] = ~0ull;
+        if (mine[e] != 0xFFFFFFFFu) {
+            const uint32_t id = s_hash[mine[e]];
+            const uint32_t fl = (s_flag[mine[e] >> 5] >> (mine[e] & 31)) & 1u;
+            const float* xv = a.x + (uint64_t)id * dim;
+            const float d = v4 ? l2_ref_order_v4(xn, xv, dim) : l2_ref_order(xn, xv, dim);
+            key[e] = ((unsigned long long)__float_as_uint(d) << 32) | (id << 1) | fl;
+        }
+    }
+    // 3. sort ascending: a bitonic network over 256 keys, two per thread
+    // (elements 2 tid and 2 tid + 1), by shuffles inside a warp and through
+    // shared memory for the three exchanges between warps
+#pragma unroll 1
+    for (uint32_t k = 2; k <= (uint32_t)kCandMax; k <<= 1) {
+#pragma unroll 1
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            const bool up = ((2u * tid) & k) == 0;
+            if (j == 1) {
+                const bool sw = (key[0] > key[1]) == up;
+                const unsigned long long t = key[0];
+                if (sw) {
+                    key[0] = key[1];
+                    key[1] = t;
+                }
+            } else {
+                unsigned long long o[2];
+                if (j < 64) {
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) o[e] = __shfl_xor_sync(0xFFFFFFFFu, key[e], j >> 1);
+                } else {
+                    s_x[2 * tid] = key[0];
+                    s_x[2 * tid + 1] = key[1];
+                    __syncthreads();
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) o[e] = s_x[(2 * tid + e) ^ j];
+                    __syncthreads();
+                }
+                const bool low = ((2u * tid) & j) == 0;  // this side keeps the smaller if up
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    if ((o[e] < key[e]) == (low == up)) key[e] = o[e];
+            }
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const uint32_t db = (uint32_t)(key[e] >> 32);
+        s_ids[2 * tid + e] = (uint32_t)key[e];
+        s_d[2 * tid + e] = key[e] == ~0ull ? CUDART_INF_F : __uint_as_float(db);
+    }
+    __syncthreads();
     uint32_t P = 0;
     {
         // valid candidates are the finite-distance prefix
@@ -488,41 +531,69 @@ __global__ void __launch_bounds__(kPruneThreads) prune_kernel(PruneArgs a) {
     }
 
     // 4. pairwise distances among the first P candidates
-    __shared__ uint64_t s_mbar;
+    __shared__ uint64_t s_mbar[2];
     __shared__ uint32_t s_tmem;
     __shared__ float s_norm[128];
-    __shared__ int s_exact;
-    if (tid == 0) s_exact = 0;
+    // 5a's decisions: bit i of row j: kept j would prune later i
+    constexpr uint32_t kOccW = (kPruneMax + 31) / 32;
+    constexpr uint32_t kRecheckCap = 1024;  // uncertain pairs listed per node
+    __shared__ uint32_t s_occ[kPruneMax][kOccW];
+    __shared__ uint16_t s_rl[kRecheckCap];  // (j << 7 | i) of uncertain pairs
+    __shared__ uint32_t s_nrl;
+    // the FP32 value of pair (j, i), in the CUDA-core path's order
+    auto fp32_pair = [&](uint32_t j, uint32_t i) {
+        const float* xj = a.x + (uint64_t)(s_ids[j] >> 1) * dim;
+        const float* xi = a.x + (uint64_t)(s_ids[i] >> 1) * dim;
+        float t = 0.f;
+        uint32_t d = 0;
+        if (v4)
+            for (; d < dim; d += 4) {
+                const float4 p = __ldg(reinterpret_cast<const float4*>(xj + d));
+                const float4 q = __ldg(reinterpret_cast<const float4*>(xi + d));
+                float df = p.x - q.x;
+                t = fmaf(df, df, t);
+                df = p.y - q.y;
+                t = fmaf(df, df, t);
+                df = p.z - q.z;
+                t = fmaf(df, df, t);
+                df = p.w - q.w;
+                t = fmaf(df, df, t);
+            }
+        for (; d < dim; ++d) {
+            const float df = xj[d] - xi[d];
+            t = fmaf(df, df, t);
+        }
+        return t;
+    };
+    for (uint32_t i = tid; i < kPruneMax; i += kPruneThreads) s_keep[i] = 0;
+    if (tid == 0) s_nrl = 0;
     if constexpr (TC != 0) {
-        // Gram matrices on the tensor cores (see tc:: above), each centred
-        // value split into BF16 hi + lo (x = hi + lo + r, |r| <= 2^-16 |x|):
-        // G~ = Ghh + Ghl + Ghl^T, two accumulators in tensor memory (columns
-        // 0.. and 128..), so the BF16 error that decides how many decisions
-        // need an FP32 re-check is 2^-16 instead of 2^-8.
-        __nv_bfloat16* op_hi = reinterpret_cast<__nv_bfloat16*>(tile);  // 128 x 128, 32 KB
-        __nv_bfloat16* op_lo = op_hi + 128 * kTileD;                      // 128 x 128, 32 KB
         if (tid < 32) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                         ::"r"(tc::smem_u32(&s_tmem)), "r"(256u));
+                         ::"r"(tc::smem_u32(&s_tmem)), "r"(128u));
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
         }
         if (tid == 0) {
-            tc::mbar_init(&s_mbar, 1);
+            tc::mbar_init(&s_mbar[0], 1);
+            tc::mbar_init(&s_mbar[1], 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem = s_tmem;
-        const float* xn = a.x + node * dim;
         const float* xr = a.x + (uint64_t)(s_ids[tid < P ? tid : 0] >> 1) * dim;
         float nrm = 0.f;  // |hi|^2 + 2 hi.lo: the Gram diagonal's form
         bool ok = true, rounded = false;
-        uint32_t chunk = 0;
-        for (uint32_t d0 = 0; d0 < dim; d0 += kTileD, ++chunk) {
+        const uint32_t chunks = (dim + kOpDims - 1) / kOpDims;
+        for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
+            const uint32_t d0 = chunk * kOpDims, buf = chunk & 1u;
+            unsigned char* op = smem + buf * kOpBytes;  // hi, then lo: 128 rows each
+            // the buffer's last MMAs must be done (chunk - 2)
+            if (chunk >= 2 && !tc::mbar_wait(&s_mbar[buf], ((chunk >> 1) - 1u) & 1u)) ok = false;
             // row tid of this chunk: x_candidate - x_node split, zero past P and dim
 #pragma unroll 2
-            for (uint32_t kc = 0; kc < kTileD / 8; ++kc) {
+            for (uint32_t kc = 0; kc < kOpDims / 8; ++kc) {
                 uint32_t wh[4], wl[4];
                 float f[8];
                 const uint32_t db = d0 + kc * 8;
@@ -557,78 +628,106 @@ __global__ void __launch_bounds__(kPruneThreads) prune_kernel(PruneArgs a) {
                     wh[e] = *reinterpret_cast<const uint32_t*>(&h);
                     wl[e] = *reinterpret_cast<const uint32_t*>(&l);
                 }
-                const uint32_t off = kc * 128 + (tid >> 3) * 2048 + (tid & 7) * 16;
-                *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(op_hi) + off) =
-                    make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(op_lo) + off) =
+                const uint32_t off = kc * 128 + (tid >> 3) * kOpSbo + (tid & 7) * 16;
+                *reinterpret_cast<uint4*>(op + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+                *reinterpret_cast<uint4*>(op + kOpBytes / 2 + off) =
                     make_uint4(wl[0], wl[1], wl[2], wl[3]);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncthreads();
             if (tid == 0) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t bh = tc::smem_u32(op_hi), bl = tc::smem_u32(op_lo);
+                const uint32_t bh = tc::smem_u32(op), bl = bh + kOpBytes / 2;
                 constexpr uint32_t idesc = tc::idesc_bf16_f32(128, kPruneMax);
 #pragma unroll
-                for (uint32_t s = 0; s < kTileD / 16; ++s) {
-                    const uint64_t dh = tc::smem_desc(bh + s * 256, 128, 2048);
-                    const uint64_t dl = tc::smem_desc(bl + s * 256, 128, 2048);
-                    const uint32_t acc = (chunk > 0 || s > 0) ? 1u : 0u;
-                    tc::mma_bf16(tmem, dh, dh, idesc, acc);          // Ghh
-                    tc::mma_bf16(tmem + 128u, dh, dl, idesc, acc);   // Ghl
+                for (uint32_t k = 0; k < kOpDims / 16; ++k) {
+                    const uint64_t dh = tc::smem_desc(bh + k * 256, 128, kOpSbo);
+                    const uint64_t dl = tc::smem_desc(bl + k * 256, 128, kOpSbo);
+                    tc::mma_bf16(tmem, dh, dh, idesc, (chunk > 0 || k > 0) ? 1u : 0u);
+                    tc::mma_bf16(tmem, dh, dl, idesc, 1u);
+                    tc::mma_bf16(tmem, dl, dh, idesc, 1u);
                 }
-                tc::commit(&s_mbar);
+                tc::commit(&s_mbar[buf]);
             }
-            // the operand tiles are rewritten next chunk: wait for these MMAs
-            if (!tc::mbar_wait(&s_mbar, chunk & 1u)) ok = false;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
         s_norm[tid] = nrm;
         // every staged value exact in BF16 and every norm below 2^23: the
         // Gram matrix (its partial sums are bounded by the norms) and the
         // distances are exact, so no decision needs a re-check
-        const int exact = !__syncthreads_or(rounded || nrm >= 8388608.0f);
-        if (tid == 0) s_exact = exact;
-        // row tid of Ghl into the pair buffer, for its transpose
-        const uint32_t w = tid >> 5;
-#pragma unroll 1
-        for (uint32_t c0 = 0; c0 < (uint32_t)kPruneMax; c0 += 16) {
-            float g[16];
-            tc::ld16(tmem + ((32u * w) << 16) + 128u + c0, g);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (tid < P)
+        const bool exact = !__syncthreads_or(rounded || nrm >= 8388608.0f);
+        // the last commit follows every MMA of the block
+        if (!tc::mbar_wait(&s_mbar[(chunks - 1) & 1u], ((chunks - 1) >> 1) & 1u)) ok = false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // 5a. every pair's occlusion decision: kept j (= tid) would prune later
+        // i when alpha^2 d(j, i) < d(node, i). The split-BF16 estimate decides
+        // unless it lies within its error bound of the threshold; then the
+        // pair is listed and its FP32 value, in the CUDA-core path's order,
+        // decides. The bound on |estimate - FP32 value|: the split's residuals
+        // (2^-15 sqrt(d) (|a| + |b|)), the missing lo.lo term (2^-15 (na +
+        // nb)), FP32 accumulation in tensor memory and in the FP32 path (about
+        // 2 D 2^-24 (na + nb) each), with a factor of 2 to spare. With sqrt(d)
+        // <= |a| + |b| a looser bound without the root clears most pairs.
+        uint32_t occ[kOccW];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) pair[tid * kPruneMax + c0 + e] = g[e];
-        }
-        __syncthreads();
-        // squared distances of row tid to the later columns: the upper
-        // triangle is rewritten while only the lower one is read
+        for (uint32_t w = 0; w < kOccW; ++w) occ[w] = 0;
+        const float rj = sqrtf(nrm);
+        const float abs_c = 2.384185791015625e-07f * (float)dim + 1.220703125e-04f;
 #pragma unroll 1
-        for (uint32_t c0 = 0; c0 < (uint32_t)kPruneMax; c0 += 16) {
-            float gh[16], gl[16];
-            tc::ld16(tmem + ((32u * w) << 16) + c0, gh);
-            tc::ld16(tmem + ((32u * w) << 16) + 128u + c0, gl);
+        for (uint32_t c0 = 0; c0 < P; c0 += 16) {
+            float g[16];
+            tc::ld16(tmem + ((32u * (tid >> 5)) << 16) + c0, g);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (tid < P) {
+            if (tid < P && c0 + 15 > tid) {
+                uint32_t bits = 0;
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    const uint32_t c = c0 + e;
-                    if (c < P && c > tid) {
-                        const float gt = __fadd_rn(__fadd_rn(gh[e], gl[e]), pair[c * kPruneMax + tid]);
-                        pair[tid * kPruneMax + c] =
-                            fmaxf(0.f, __fsub_rn(__fadd_rn(nrm, s_norm[c]), 2.f * gt));
+                    const uint32_t i = c0 + e;
+                    if (i <= tid || i >= P) continue;
+                    const float ni = s_norm[i], di = s_d[i];
+                    const float dji = fmaxf(0.f, __fsub_rn(__fadd_rn(nrm, ni), 2.f * g[e]));
+                    if (!exact) {
+                        const float ri = sqrtf(ni);
+                        const float off = fabsf(a.alpha2 * dji - di), base = abs_c * (ni + nrm);
+                        if (off <= a.alpha2 * 1.001f * (6.103515625e-05f * (ri + rj) * (ri + rj) * 1.001f + base)) {
+                            const float err = 6.103515625e-05f * sqrtf(dji) * (ri + rj) + base;
+                            if (off <= a.alpha2 * err) {
+                                // listed, and re-checked below by all threads
+                                // at once; past the list's end, here
+                                const uint32_t slot = atomicAdd(&s_nrl, 1u);
+                                if (slot < kRecheckCap) {
+                                    s_rl[slot] = (uint16_t)((tid << 7) | i);
+                                    continue;
+                                }
+                                if (a.rechecks) atomicAdd(a.rechecks, 1ull);
+                                if (a.alpha2 * fp32_pair(tid, i) < di) bits |= 1u << e;
+                                continue;
+                            }
+                        }
                     }
+                    if (a.alpha2 * dji < di) bits |= 1u << e;
                 }
+#pragma unroll
+                for (uint32_t w = 0; w < kOccW; ++w)
+                    if ((c0 >> 5) == w) occ[w] |= bits << (c0 & 31u);
             }
         }
+        if (tid < kPruneMax)
+#pragma unroll
+            for (uint32_t w = 0; w < kOccW; ++w) s_occ[tid][w] = occ[w];
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         if (tid < 32) {
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u));
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128u));
         }
         if (!ok && tid == 0 && a.err) atomicOr(a.err, 1u);
+        const uint32_t nrl = min(s_nrl, kRecheckCap);
+        for (uint32_t t = tid; t < nrl; t += kPruneThreads) {
+            const uint32_t j = s_rl[t] >> 7, i = s_rl[t] & 127u;
+            if (a.alpha2 * fp32_pair(j, i) < s_d[i]) atomicOr(&s_occ[j][i >> 5], 1u << (i & 31));
+        }
+        if (a.rechecks && tid == 0 && nrl) atomicAdd(a.rechecks, (unsigned long long)nrl);
+        __syncthreads();
     } else {
-        if (tid < 128) s_norm[tid] = 0.f;
         // 4. pairwise distances among the first P candidates, tiled over dims.
         // Thread t owns pairs p = t + kPruneThreads * s of the strict upper
         // triangle in row-major order.
@@ -683,84 +782,17 @@ __global__ void __launch_bounds__(kPruneThreads) prune_kernel(PruneArgs a) {
             if (p < npairs) pair[(pab[s] & 0xFFFFu) * kPruneMax + (pab[s] >> 16)] = acc[s];
         }
     }
-    // 5a. every pair's occlusion decision at once: kept j would prune later i
-    // when alpha^2 d(j, i) < d(node, i). On the tensor-core path the split-
-    // BF16 estimate decides unless it lies within its error bound of the
-    // threshold; then the FP32 value, in the same order as the CUDA-core path,
-    // decides. A decision does not depend on which candidates the greedy pass
-    // keeps, so all pairs are decided in parallel, one bit each, with no
-    // barrier per kept neighbour (the narrow bound leaves few re-checks, and
-    // they run spread over the whole block).
-    constexpr uint32_t kOccW = (kPruneMax + 31) / 32;
-    constexpr uint32_t kRecheckCap = 1024;  // uncertain pairs listed per node
-    __shared__ uint32_t s_occ[kPruneMax][kOccW];
-    __shared__ uint16_t s_rl[kRecheckCap];   // (j << 7 | i) of uncertain pairs
-    __shared__ uint32_t s_nrl;
-    for (uint32_t i = tid; i < (uint32_t)kPruneMax * kOccW; i += kPruneThreads)
-        (&s_occ[0][0])[i] = 0;
-    for (uint32_t i = tid; i < kPruneMax; i += kPruneThreads) s_keep[i] = 0;
-    if (tid == 0) s_nrl = 0;
-    __syncthreads();
-    // the FP32 value of pair (j, i), in the CUDA-core path's order
-    auto fp32_pair = [&](uint32_t j, uint32_t i) {
-        const float* xj = a.x + (uint64_t)(s_ids[j] >> 1) * dim;
-        const float* xi = a.x + (uint64_t)(s_ids[i] >> 1) * dim;
-        float t = 0.f;
-        uint32_t d = 0;
-        if (v4)
-            for (; d < dim; d += 4) {
-                const float4 p = __ldg(reinterpret_cast<const float4*>(xj + d));
-                const float4 q = __ldg(reinterpret_cast<const float4*>(xi + d));
-                float df = p.x - q.x;
-                t = fmaf(df, df, t);
-                df = p.y - q.y;
-                t = fmaf(df, df, t);
-                df = p.z - q.z;
-                t = fmaf(df, df, t);
-                df = p.w - q.w;
-                t = fmaf(df, df, t);
-            }
-        for (; d < dim; ++d) {
-            const float df = xj[d] - xi[d];
-            t = fmaf(df, df, t);
+    // 5a for the FP32 path: all pairs decided in parallel, one bit each (a
+    // decision does not depend on which candidates the greedy pass keeps)
+    if constexpr (TC == 0) {
+        for (uint32_t i = tid; i < (uint32_t)kPruneMax * kOccW; i += kPruneThreads)
+            (&s_occ[0][0])[i] = 0;
+        __syncthreads();
+        for (uint32_t e = tid; e < P * P; e += kPruneThreads) {
+            const uint32_t j = e / P, i = e % P;
+            if (i > j && a.alpha2 * pair[j * kPruneMax + i] < s_d[i])
+                atomicOr(&s_occ[j][i >> 5], 1u << (i & 31));
         }
-        return t;
-    };
-    for (uint32_t e = tid; e < P * P; e += kPruneThreads) {
-        const uint32_t j = e / P, i = e % P;
-        if (i <= j) continue;
-        float dji = pair[j * kPruneMax + i];
-        if (TC && !s_exact) {
-            // bound on |estimate - FP32 value|: the split's residuals
-            // (2^-15 sqrt(d) (|a| + |b|)), the missing lo.lo term
-            // (2^-15 (na + nb)), FP32 accumulation in tensor memory and in the
-            // FP32 path (about 2 D 2^-24 (na + nb) each), with a factor of 2 to spare
-            const float ni = s_norm[i], nj = s_norm[j];
-            const float err = 6.103515625e-05f * sqrtf(fmaxf(dji, 0.f)) * (sqrtf(ni) + sqrtf(nj)) +
-                              (2.384185791015625e-07f * (float)dim + 1.220703125e-04f) * (ni + nj);
-            if (fabsf(a.alpha2 * dji - s_d[i]) <= a.alpha2 * err) {
-                // listed, and re-checked below by all threads at once (a
-                // re-check in this loop would keep its warp's other lanes
-                // idle for the whole row); past the list's end, here
-                const uint32_t slot = atomicAdd(&s_nrl, 1u);
-                if (slot < kRecheckCap) {
-                    s_rl[slot] = (uint16_t)((j << 7) | i);
-                    continue;
-                }
-                dji = fp32_pair(j, i);
-                if (a.rechecks) atomicAdd(a.rechecks, 1ull);
-            }
-        }
-        if (a.alpha2 * dji < s_d[i]) atomicOr(&s_occ[j][i >> 5], 1u << (i & 31));
-    }
-    __syncthreads();
-    if (TC) {
-        const uint32_t nrl = min(s_nrl, kRecheckCap);
-        for (uint32_t t = tid; t < nrl; t += kPruneThreads) {
-            const uint32_t j = s_rl[t] >> 7, i = s_rl[t] & 127u;
-            if (a.alpha2 * fp32_pair(j, i) < s_d[i]) atomicOr(&s_occ[j][i >> 5], 1u << (i & 31));
-        }
-        if (a.rechecks && tid == 0 && nrl) atomicAdd(a.rechecks, (unsigned long long)nrl);
         __syncthreads();
     }
 
@@ -858,9 +890,9 @@ __global__ void __launch_bounds__(kPruneThreads) prune_kernel(PruneArgs a) {
     }
 }
 
-size_t prune_smem_bytes(int tc) {
-    const size_t tile = tc ? (size_t)128 * kTileD : (size_t)(kPruneMax + 1) * (kTileD + 1);
-    return sizeof(float) * (tile + (size_t)kPruneMax * kPruneMax);
+size_t prune_smem_bytes(int tc, uint32_t dim) {
+    if (tc) return (size_t)kOpBytes * (dim > kOpDims ? 2 : 1);
+    return sizeof(float) * ((size_t)(kPruneMax + 1) * (kTileD + 1) + (size_t)kPruneMax * kPruneMax);
 }
 
 // Reverse lists as CSR, deterministic: pair (target, source) for every kept
@@ -889,7 +921,7 @@ __global__ void segment_kernel(const uint32_t* __restrict__ keys, uint64_t total
 }
 
 cudaError_t launch_prune(const PruneArgs& a, uint64_t nodes, cudaStream_t st) {
-    const size_t smem = prune_smem_bytes(a.pair_tc);
+    const size_t smem = prune_smem_bytes(a.pair_tc, a.dim);
     auto k = a.pair_tc ? prune_kernel<1> : prune_kernel<0>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -85,8 +85,12 @@ struct FsSearchArgs {
 
 __host__ __device__ inline uint32_t al16(uint64_t x) { return (uint32_t)((x + 15) & ~15ull); }
 
+// Slots of the sorted buffer: whole rows of 32, one slot past efcap at least
+// (it holds +inf).
+__host__ __device__ inline uint32_t fs_slots(uint32_t efcap) { return (efcap + 32u) & ~31u; }
+
 struct FsWarpLayout {
-    uint32_t row, bar, qs, lut, sb_a, sb_b, rb, rcopy, vis, total;
+    uint32_t row, bar, qs, lut, sb, rb, rcopy, vis, total;
 };
 
 __host__ __device__ inline FsWarpLayout fs_layout(uint32_t dim, uint32_t P, uint64_t row_bytes,
@@ -101,10 +105,8 @@ __host__ __device__ inline FsWarpLayout fs_layout(uint32_t dim, uint32_t P, uint
     o += al16(4ull * ((dim + 15) & ~15u));
     L.lut = o;
     o += al16(4ull * P);
-    L.sb_a = o;
-    o += al16(8ull * (efcap + 1));
-    L.sb_b = o;
-    o += al16(8ull * (efcap + 1));
+    L.sb = o;
+    o += 8u * fs_slots(efcap);
     L.rb = o;
     o += al16(8ull * (kcap + 1));
     L.rcopy = o;
@@ -248,17 +250,18 @@ __device__ __forceinline__ float exact_l2(const float* q, const float* v, uint32
     return r;
 }
 
-// Number of entries of the ascending d[0, n) strictly below y.
+// Number of entries of the ascending d[0, n) strictly below y, n > 0: no
+// branches; the slots past the last entry hold +inf, so n is the array's
+// length.
 __device__ __forceinline__ uint32_t count_below(const float* d, uint32_t n, float y) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (d[mid] < y)
-            lo = mid + 1;
-        else
-            hi = mid;
+    const float* p = d;
+#pragma unroll 1
+    while (n > 1) {  // warp-uniform
+        const uint32_t half = n >> 1;
+        if (p[half - 1] < y) p += half;
+        n -= half;
     }
-    return lo;
+    return (uint32_t)(p - d) + (*p < y ? 1u : 0u);
 }
 
 // ResultBuffer::insert (utils/buffer.hpp:86-97): capacity k; a distance above
@@ -267,7 +270,7 @@ __device__ __forceinline__ uint32_t count_below(const float* d, uint32_t n, floa
 __device__ __forceinline__ void result_insert(float* rd, uint32_t* ri, uint32_t& rsize, uint32_t k,
                                               uint32_t id, float y, int lane) {
     if (k == 0 || (rsize == k && y > rd[rsize - 1])) return;
-    const uint32_t pos = count_below(rd, rsize, y);
+    const uint32_t pos = rsize ? count_below(rd, rsize, y) : 0u;
     // shift [pos, rsize) up by one (into the k + 1 slots), from the top
     for (int base = (int)((rsize - 1) & ~31u); rsize > pos && base >= (int)(pos & ~31u); base -= 32) {
         const uint32_t x = (uint32_t)base + lane;
@@ -305,9 +308,9 @@ __global__ void __launch_bounds__(256, 4) fs_search_kernel(FsSearchArgs a) {
     uint64_t* bar = reinterpret_cast<uint64_t*>(wb + L.bar);
     float* qs = reinterpret_cast<float*>(wb + L.qs);
     uint8_t* lut = wb + L.lut;
-    float* sbd[2] = {reinterpret_cast<float*>(wb + L.sb_a), reinterpret_cast<float*>(wb + L.sb_b)};
-    uint32_t* sbi[2] = {reinterpret_cast<uint32_t*>(sbd[0] + (a.efcap + 1)),
-                        reinterpret_cast<uint32_t*>(sbd[1] + (a.efcap + 1))};
+    const uint32_t slots = fs_slots(a.efcap);
+    float* sd = reinterpret_cast<float*>(wb + L.sb);  // sorted buffer: distances
+    uint32_t* si = reinterpret_cast<uint32_t*>(sd + slots);  // and ids
     float* rd = reinterpret_cast<float*>(wb + L.rb);
     uint32_t* ri = reinterpret_cast<uint32_t*>(rd + (a.kcap + 1));
     uint32_t* rcopy = reinterpret_cast<uint32_t*>(wb + L.rcopy);
@@ -422,9 +425,8 @@ __global__ void __launch_bounds__(256, 4) fs_search_kernel(FsSearchArgs a) {
         __syncwarp();
 
         // ---- search_qg (qg.hpp:252-287) ----
-        int cb = 0;  // current sorted buffer
-        float* sd = sbd[0];
-        uint32_t* si = sbi[0];
+        for (uint32_t i = lane; i < slots; i += 32) sd[i] = CUDART_INF_F;
+        __syncwarp();
         if (lane == 0) {
             sd[0] = CUDART_MAX_NORMAL_F;  // FLT_MAX
             si[0] = a.entry;
@@ -433,6 +435,30 @@ __global__ void __launch_bounds__(256, 4) fs_search_kernel(FsSearchArgs a) {
         uint32_t size = 1, cur = 0, rsize = 0, nvis = 0;
         uint32_t pops = 0, exact = 0, upd = 0;
         bool fail = false, overflow = false;
+        // The row buffer: at most one copy is in flight, of node `coming`'s row
+        // (kEmpty: none); every copy is waited for once.
+        uint32_t coming = kEmpty;
+        auto start = [&](uint32_t id) {
+            coming = id;
+            __syncwarp();
+            if (lane == 0)
+                bulk_row_copy(row, a.rows + (size_t)id * a.row_bytes, (uint32_t)a.row_bytes, bar);
+        };
+        // Waits for the copy in flight; false (and the error is reported) when
+        // it did not complete in time.
+        auto arrive = [&]() -> bool {
+            coming = kEmpty;
+            bool ok = mbar_wait(bar, phase);
+            if (!ok) {
+                if (lane == 0) {
+                    atomicOr(a.err, kFsErrCopy);
+                    atomicCAS(a.err + 1, kNoId, (uint32_t)qi);
+                }
+                mbar_wait(bar, phase);
+            }
+            phase ^= 1u;
+            return ok;
+        };
 
         while (cur < size && !fail) {
             // SearchBuffer::pop (buffer.hpp:52-60)
@@ -458,23 +484,15 @@ __global__ void __launch_bounds__(256, 4) fs_search_kernel(FsSearchArgs a) {
                 overflow = true;
                 break;
             }
-            // the next unchecked node is the likely next pop: ask L2 for its row
+            // the node after it in the buffer: ask L2 for its row
             if (lane == 0 && cur < size)
                 l2_prefetch_row(a.rows + (size_t)si[cur] * a.row_bytes, (uint32_t)a.row_bytes);
-            // the popped node's row into shared memory
-            __syncwarp();
-            if (lane == 0)
-                bulk_row_copy(row, a.rows + (size_t)u * a.row_bytes, (uint32_t)a.row_bytes, bar);
-            if (!mbar_wait(bar, phase)) {
-                // the copy never completed: report, wait once more, give up the warp
-                if (lane == 0) {
-                    atomicOr(a.err, kFsErrCopy);
-                    atomicCAS(a.err + 1, kNoId, (uint32_t)qi);
-                }
-                mbar_wait(bar, phase);
-                return;
+            // the popped node's row into shared memory (mostly it is on its way)
+            if (coming != u) {
+                if (coming != kEmpty && !arrive()) return;
+                start(u);
             }
-            phase ^= 1u;
+            if (!arrive()) return;
             const float* vec = reinterpret_cast<const float*>(row);
             const uint8_t* codes = row + a.off_codes;
             const float* fac = reinterpret_cast<const float*>(row + a.off_fac);
@@ -512,9 +530,9 @@ __global__ void __launch_bounds__(256, 4) fs_search_kernel(FsSearchArgs a) {
                         if (PB < 16 && e >= 2) break;
 #pragma unroll
                         for (int bi = 0; bi < 4; ++bi) {
-                            const uint32_t byte = (cw[e] >> (8 * bi)) & 0xFFu;
-                            const uint8_t* gl = lg + 32 * (4 * e + bi);
-                            s += gl[byte & 15u] + gl[16 + (byte >> 4)];
+                            const uint32_t lo4 = (cw[e] >> (8 * bi)) & 15u;
+                            const uint32_t hi4 = bi < 3 ? (cw[e] >> (8 * bi + 4)) & 15u : cw[e] >> 28;
+                            s += lg[32 * (4 * e + bi) + lo4] + lg[32 * (4 * e + bi) + 16 + hi4];
                         }
                     }
                 }
@@ -544,107 +562,137 @@ __global__ void __launch_bounds__(256, 4) fs_search_kernel(FsSearchArgs a) {
             // goes in exactly when fewer than ef of everything inserted so far
             // lies strictly below it; the buffer holds the ef smallest of
             // those, so that is #{buffer < y_j} + #{earlier candidates < y_j}.
-            uint32_t below[DEGW], pc[DEGW];
-            bool acc[DEGW];
+            // An inserted value goes before equal ones already there, so the
+            // merged order is by distance, later candidates first.
+            uint32_t below[DEGW], pc[DEGW], pos[DEGW];
+            unsigned cm[DEGW];
+            uint32_t any = 0;
 #pragma unroll
             for (int w = 0; w < DEGW; ++w) {
                 // a full buffer whose largest value lies below y_j already
                 // holds ef values under it: j cannot go in, and it lies above
                 // every candidate that can, so it counts for none of them
                 cand[w] = cand[w] && (size < ef || y[w] <= sd[size - 1]);
-                below[w] = cand[w] ? count_below(sd, size, y[w]) : 0u;
+                cm[w] = __ballot_sync(kFull, cand[w]);
+                any |= cm[w];
             }
-#pragma unroll
-            for (int w = 0; w < DEGW; ++w) {
-                uint32_t c = 0;
-#pragma unroll
-                for (int w2 = 0; w2 <= w; ++w2) {
-                    unsigned bm = __ballot_sync(kFull, cand[w2]);  // warp-uniform loop
-                    while (bm) {
-                        const int s = __ffs(bm) - 1;
-                        bm &= bm - 1;
-                        const float ys = __shfl_sync(kFull, y[w2], s);
-                        c += ((w2 < w || s < lane) && ys < y[w]) ? 1u : 0u;
-                    }
-                }
-                pc[w] = c;
-                acc[w] = cand[w] && below[w] + c < ef;
-            }
-            unsigned am[DEGW];
-            uint32_t m = 0;
-#pragma unroll
-            for (int w = 0; w < DEGW; ++w) {
-                am[w] = __ballot_sync(kFull, acc[w]);
-                m += __popc(am[w]);
-            }
-            if (m > 0) {
-                // merged order: distance ascending; an inserted value goes
-                // before equal ones already there, so later candidates first
-                uint32_t pos[DEGW];
+            if (any) {
 #pragma unroll
                 for (int w = 0; w < DEGW; ++w) {
-                    uint32_t c = 0;
+                    below[w] = cm[w] ? count_below(sd, slots, y[w]) : 0u;
+                    pc[w] = pos[w] = 0;
+                }
+                // one pass over the candidates: the earlier ones below this
+                // lane's (pc), and those that go ahead of it (pos)
 #pragma unroll
-                    for (int w2 = 0; w2 < DEGW; ++w2) {
-                        unsigned bm = am[w2];
-                        while (bm) {
+                for (int w2 = 0; w2 < DEGW; ++w2)
+#pragma unroll 1
+                    for (unsigned bm = cm[w2]; bm; bm &= bm - 1) {
+                        const int s = __ffs(bm) - 1;
+                        const float ys = __shfl_sync(kFull, y[w2], s);
+#pragma unroll
+                        for (int w = 0; w < DEGW; ++w) {
+                            const bool early = w2 < w || (w2 == w && s < lane);
+                            const bool late = w2 > w || (w2 == w && s > lane);
+                            const bool lo = ys < y[w];
+                            pc[w] += lo && early ? 1u : 0u;
+                            pos[w] += lo || (late && ys == y[w]) ? 1u : 0u;
+                        }
+                    }
+                bool acc[DEGW];
+                unsigned am[DEGW];
+                uint32_t m = 0;
+                bool all = true;
+#pragma unroll
+                for (int w = 0; w < DEGW; ++w) {
+                    acc[w] = cand[w] && below[w] + pc[w] < ef;
+                    am[w] = __ballot_sync(kFull, acc[w]);
+                    all = all && am[w] == cm[w];
+                    m += __popc(am[w]);
+                }
+                if (!all) {  // rare: only the accepted ones are placed
+#pragma unroll
+                    for (int w = 0; w < DEGW; ++w) pos[w] = 0;
+#pragma unroll
+                    for (int w2 = 0; w2 < DEGW; ++w2)
+#pragma unroll 1
+                        for (unsigned bm = am[w2]; bm; bm &= bm - 1) {
                             const int s = __ffs(bm) - 1;
-                            bm &= bm - 1;
                             const float ys = __shfl_sync(kFull, y[w2], s);
-                            const int js = w2 * 32 + s, jj = w * 32 + lane;
-                            c += (ys < y[w] || (ys == y[w] && js > jj)) ? 1u : 0u;
+#pragma unroll
+                            for (int w = 0; w < DEGW; ++w)
+                                pos[w] += ys < y[w] || (ys == y[w] && w2 * 32 + s > w * 32 + lane) ? 1u : 0u;
                         }
-                    }
-                    pos[w] = below[w] + c;
                 }
-                float* nd = sbd[cb ^ 1];
-                uint32_t* ni = sbi[cb ^ 1];
-                const uint32_t nsize = min(size + m, ef);
-                uint32_t ncur = kEmpty;
-                // the old entries move up by the inserted values at or below them
-                for (uint32_t x0 = 0; x0 < size; x0 += 32) {
-                    const uint32_t x = x0 + lane;
-                    float dx = 0.f;
-                    uint32_t ix = 0, sh = 0;
-                    if (x < size) {
-                        dx = sd[x];
-                        ix = si[x];
+                if (m > 0) {
+                    const uint32_t nsize = min(size + m, ef);
+                    uint32_t first = kEmpty, ahead = 0;  // the first new place; those before `cur`
+#pragma unroll
+                    for (int w = 0; w < DEGW; ++w) {
+                        pos[w] += below[w];
+                        if (acc[w]) first = min(first, pos[w]);
+                        ahead += __popc(__ballot_sync(kFull, acc[w] && below[w] <= cur));
+                    }
+                    const uint32_t fmine = first;
+                    first = __reduce_min_sync(kFull, first);
+                    // the next pop is the first unchecked entry; start on its
+                    // row before the buffer is moved, unless it was expanded
+                    {
+                        uint32_t nid = cur < size ? si[cur] : kEmpty;
+                        if (cur >= size || first < cur + ahead) {
+                            const int s = __ffs(__ballot_sync(kFull, fmine == first)) - 1;
+                            uint32_t mineid = 0;
+#pragma unroll
+                            for (int w = 0; w < DEGW; ++w)
+                                if (acc[w] && pos[w] == first) mineid = id[w];
+                            nid = __shfl_sync(kFull, mineid, s);
+                        }
+                        if (nid != kEmpty && !vis_has(vis, a.vbits, nid)) start(nid);
+                    }
+                    // rows of 32 slots from the top: the slots that accepted
+                    // ones take as a bit mask; every other slot gets the old
+                    // entry as many places down as accepted ones lie below it
+                    uint32_t under = m;
+#pragma unroll 1
+                    for (int rr = (int)((size + m - 1) >> 5); rr >= (int)(first >> 5); --rr) {
+                        uint32_t bits = 0;
+#pragma unroll
+                        for (int w = 0; w < DEGW; ++w)
+                            bits |= acc[w] && (int)(pos[w] >> 5) == rr ? 1u << (pos[w] & 31u) : 0u;
+                        const unsigned taken = __reduce_or_sync(kFull, bits);
+                        under -= __popc(taken);
+                        const uint32_t x = (uint32_t)rr * 32 + lane;
+                        const uint32_t sh = under + __popc(taken & ((1u << lane) - 1u));
+                        const bool mv = sh > 0 && x < nsize && !((taken >> lane) & 1u);
+                        float xd = 0.f;
+                        uint32_t xi = 0;
+                        if (mv) {
+                            xd = sd[x - sh];
+                            xi = si[x - sh];
+                        }
+                        __syncwarp();
+                        if (mv) {
+                            sd[x] = xd;
+                            si[x] = xi;
+                        }
+                        __syncwarp();
                     }
 #pragma unroll
-                    for (int w2 = 0; w2 < DEGW; ++w2) {
-                        unsigned bm = am[w2];
-                        while (bm) {
-                            const int s = __ffs(bm) - 1;
-                            bm &= bm - 1;
-                            sh += __shfl_sync(kFull, y[w2], s) <= dx ? 1u : 0u;
+                    for (int w = 0; w < DEGW; ++w)
+                        if (acc[w] && pos[w] < nsize) {
+                            sd[pos[w]] = y[w];
+                            si[pos[w]] = id[w];
                         }
-                    }
-                    const uint32_t np = x + sh;
-                    if (x < size && np < nsize) {
-                        nd[np] = dx;
-                        ni[np] = ix;
-                        if (!(ix & kChecked)) ncur = min(ncur, np);
-                    }
+                    __syncwarp();
+                    cur = min(min(cur < size ? cur + ahead : kEmpty, first), nsize);
+                    size = nsize;
                 }
-#pragma unroll
-                for (int w = 0; w < DEGW; ++w)
-                    if (acc[w] && pos[w] < nsize) {
-                        nd[pos[w]] = y[w];
-                        ni[pos[w]] = id[w];
-                        ncur = min(ncur, pos[w]);
-                    }
-                ncur = __reduce_min_sync(kFull, ncur);
-                __syncwarp();
-                cb ^= 1;
-                sd = nd;
-                si = ni;
-                size = nsize;
-                cur = min(ncur, size);
             }
             // ResultBuffer::insert of the popped node (qg.hpp:285)
             result_insert(rd, ri, rsize, k, u, sqr_y, lane);
         }
 
+        if (coming != kEmpty && !arrive()) return;
         // update_results (qg.hpp:395-418): fewer than k results
         if (!fail && !overflow && rsize < k) {
             for (uint32_t t = lane; t <= k; t += 32) rcopy[t] = t < rsize ? ri[t] : 0u;

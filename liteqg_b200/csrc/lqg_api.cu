@@ -248,7 +248,13 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         ra.nspill = w.d_ctl + kCtlSpilled;
         ra.rlog_cap = std::max(1024u, 16u * b.ef0);
         ra.replay_all = t.replay_all;
-        ra.acap = 32u * (uint32_t)RE;
+        // sorted pool of the batch kernels: ef, an expansion's 32 candidates and
+        // a row for ties with the bound. (Without that row one tie kept past an
+        // ef that is a multiple of 32 and 32 accepted candidates overflow it, as
+        // happens while a search descends, and the query goes to the exact
+        // kernel: one such query of 2,000 took the batch from 2.5 to 6.2 ms at
+        // 100k x 768, ef 128.)
+        ra.acap = 32u * (uint32_t)RE + 32u;
         ra.lazy = lazy ? 1u : 0u;
         const int64_t chunk = std::min<int64_t>(
             b.m, std::max<int64_t>(1024, (int64_t(1) << 30) / ((int64_t)ra.rlog_cap * 16)));

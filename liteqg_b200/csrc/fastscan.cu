@@ -1106,11 +1106,6 @@ lqg_status fs_run(lqg_index* ix, Workspace& w, const float* q, int64_t m, const 
         a.qhead = w.d_ctl + (round ? kCtlHeapHead : kCtlFastHead);
         a.retry = w.d_flagged;
         a.nretry = w.d_ctl + kCtlFlagged;
-        if (round == 0) {
-            LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlFastHead, 0, 4, st));
-            LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlHeapHead, 0, 4, st));
-            LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlFlagged, 0, 4, st));
-        }
         kern<<<(unsigned)blocks, warps * 32, smem, st>>>(a);
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "FastScan search launch");
@@ -1121,10 +1116,7 @@ lqg_status fs_run(lqg_index* ix, Workspace& w, const float* q, int64_t m, const 
     return LQG_OK;
 }
 
-lqg_status fs_status(Workspace& w, cudaStream_t st) {
-    uint32_t ctl[kCtlWords];
-    LQG_CUDA(cudaMemcpyAsync(ctl, w.d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st));
-    LQG_CUDA(cudaStreamSynchronize(st));
+lqg_status fs_status_of(const uint32_t* ctl) {
     const uint32_t e = ctl[kCtlErr];
     if (e & lqg::kFsErrCopy)
         return fail(LQG_ERR_CUDA, "a FastScan row copy did not complete (query " +
@@ -1137,6 +1129,13 @@ lqg_status fs_status(Workspace& w, cudaStream_t st) {
                                           std::to_string(ctl[kCtlErrQuery]) +
                                           "; its ids are LQG_NO_ID)");
     return LQG_OK;
+}
+
+lqg_status fs_status(Workspace& w, cudaStream_t st) {
+    uint32_t ctl[kCtlWords];
+    LQG_CUDA(cudaMemcpyAsync(ctl, w.d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st));
+    LQG_CUDA(cudaStreamSynchronize(st));
+    return fs_status_of(ctl);
 }
 
 }  // namespace
@@ -1329,16 +1328,16 @@ LQG_API lqg_status lqg_fs_search_batch(lqg_index* ix, const float* queries, int6
     if (k && (s = grow(w.d_kq, w.cap_kq, (size_t)m)) != LQG_OK) return s;
     if (ef && (s = grow(w.d_efq, w.cap_efq, (size_t)m)) != LQG_OK) return s;
     if (stats && (s = grow(w.d_stats, w.cap_stats, (size_t)m * 4)) != LQG_OK) return s;
-    LQG_CUDA(cudaMemcpyAsync(w.d_q, queries, (size_t)m * ix->dim * 4, cudaMemcpyHostToDevice, st));
-    if (k) LQG_CUDA(cudaMemcpyAsync(w.d_kq, k, m * 4, cudaMemcpyHostToDevice, st));
-    if (ef) LQG_CUDA(cudaMemcpyAsync(w.d_efq, ef, m * 4, cudaMemcpyHostToDevice, st));
+    if ((s = copy_in(w, w.d_q, queries, (size_t)m * ix->dim * 4, st)) != LQG_OK) return s;
+    if (k && (s = copy_in(w, w.d_kq, k, m * 4, st)) != LQG_OK) return s;
+    if (ef && (s = copy_in(w, w.d_efq, ef, m * 4, st)) != LQG_OK) return s;
     s = fs_run(ix, w, w.d_q, m, k ? w.d_kq : nullptr, k0, ef ? w.d_efq : nullptr, efb, w.d_ids,
                kstride, stats ? w.d_stats : nullptr, st, m == 1);
     if (s != LQG_OK) return s;
-    LQG_CUDA(cudaMemcpyAsync(ids, w.d_ids, (size_t)m * kstride * 4, cudaMemcpyDeviceToHost, st));
-    if (stats)
-        LQG_CUDA(cudaMemcpyAsync(stats, w.d_stats, (size_t)m * 16, cudaMemcpyDeviceToHost, st));
-    return fs_status(w, st);
+    if ((s = fetch_ctl(w, std::max<size_t>(kstride, 4u) * (size_t)m * 4, st)) != LQG_OK) return s;
+    if ((s = copy_out(w, ids, w.d_ids, (size_t)m * kstride * 4, st)) != LQG_OK) return s;
+    if (stats && (s = copy_out(w, stats, w.d_stats, (size_t)m * 16, st)) != LQG_OK) return s;
+    return fs_status_of(w.stage.ctl());
 }
 
 LQG_API lqg_status lqg_selftest_bounded_wait(int device, uint32_t tries, uint32_t* timed_out) {

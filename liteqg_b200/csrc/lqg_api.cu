@@ -26,6 +26,11 @@ namespace lqg_host {
 
 namespace {
 thread_local std::string g_last_error;
+
+// Control words before a batch: zero, and no failing query.
+__global__ void reset_ctl_kernel(uint32_t* ctl) {
+    ctl[threadIdx.x] = threadIdx.x == kCtlErrQuery ? 0xFFFFFFFFu : 0u;
+}
 }  // namespace
 
 lqg_status fail(lqg_status s, const std::string& msg) {
@@ -187,8 +192,8 @@ SearchArgs base_args(const lqg_index* ix, const Workspace& w, const BatchSpec& b
 }
 
 lqg_status reset_ctl(Workspace& w, cudaStream_t st) {
-    LQG_CUDA(cudaMemsetAsync(w.d_ctl, 0, kCtlWords * sizeof(uint32_t), st));
-    LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlErrQuery, 0xFF, sizeof(uint32_t), st));
+    reset_ctl_kernel<<<1, kCtlWords, 0, st>>>(w.d_ctl);
+    LQG_CUDA(cudaGetLastError());
     return LQG_OK;
 }
 
@@ -524,9 +529,9 @@ lqg_status search_host(lqg_index* ix, Workspace& w, const float* queries, int64_
         if ((s = grow(w.d_pool_ids, w.cap_pool_ids, (size_t)m * pstride)) != LQG_OK) return s;
         if ((s = grow(w.d_pool_d, w.cap_pool_d, (size_t)m * pstride)) != LQG_OK) return s;
     }
-    LQG_CUDA(cudaMemcpyAsync(w.d_q, queries, (size_t)m * ix->dim * 4, cudaMemcpyHostToDevice, st));
-    if (k) LQG_CUDA(cudaMemcpyAsync(w.d_kq, k, m * 4, cudaMemcpyHostToDevice, st));
-    if (ef) LQG_CUDA(cudaMemcpyAsync(w.d_efq, ef, m * 4, cudaMemcpyHostToDevice, st));
+    if ((s = copy_in(w, w.d_q, queries, (size_t)m * ix->dim * 4, st)) != LQG_OK) return s;
+    if (k && (s = copy_in(w, w.d_kq, k, m * 4, st)) != LQG_OK) return s;
+    if (ef && (s = copy_in(w, w.d_efq, ef, m * 4, st)) != LQG_OK) return s;
     BatchSpec b{w.d_q,
                 m,
                 k ? w.d_kq : nullptr,
@@ -541,16 +546,15 @@ lqg_status search_host(lqg_index* ix, Workspace& w, const float* queries, int64_
                 stats ? w.d_stats : nullptr,
                 st};
     if ((s = run_batch(ix, w, b, false)) != LQG_OK) return s;
-    LQG_CUDA(cudaMemcpyAsync(ids, w.d_ids, (size_t)m * kstride * 4, cudaMemcpyDeviceToHost, st));
+    const size_t most = std::max<size_t>(std::max(kstride, pool_ids ? pstride : 0u), 4u) * (size_t)m * 4;
+    if ((s = fetch_ctl(w, most, st)) != LQG_OK) return s;
+    if ((s = copy_out(w, ids, w.d_ids, (size_t)m * kstride * 4, st)) != LQG_OK) return s;
     if (pool_ids) {
-        LQG_CUDA(cudaMemcpyAsync(pool_ids, w.d_pool_ids, (size_t)m * pstride * 4,
-                                 cudaMemcpyDeviceToHost, st));
-        LQG_CUDA(cudaMemcpyAsync(pool_d, w.d_pool_d, (size_t)m * pstride * 4,
-                                 cudaMemcpyDeviceToHost, st));
+        if ((s = copy_out(w, pool_ids, w.d_pool_ids, (size_t)m * pstride * 4, st)) != LQG_OK) return s;
+        if ((s = copy_out(w, pool_d, w.d_pool_d, (size_t)m * pstride * 4, st)) != LQG_OK) return s;
     }
-    if (stats)
-        LQG_CUDA(cudaMemcpyAsync(stats, w.d_stats, (size_t)m * 16, cudaMemcpyDeviceToHost, st));
-    return read_status(w, st);
+    if (stats && (s = copy_out(w, stats, w.d_stats, (size_t)m * 16, st)) != LQG_OK) return s;
+    return status_of(w.stage.ctl());
 }
 
 }  // namespace lqg_host

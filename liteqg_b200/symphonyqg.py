@@ -146,13 +146,16 @@ class Index:
                     raise ValueError("per-query ef must have one value per query row")
                 ef0 = int(ef_arr.max()) if m else 1
         kstride = max(k, 1)
-        ids = np.full((m, kstride), LQG_NO_ID, dtype=np.uint32)
+        # every slot of these is written by the call
+        ids = np.empty((m, kstride), dtype=np.uint32)
+        if k == 0:
+            ids.fill(LQG_NO_ID)
         pstride = 0
         pool_ids = pool_d = None
         if return_pool:
             pstride = int(ef0 if ef is not None else self.get_ef())
-            pool_ids = np.full((m, pstride), LQG_NO_ID, dtype=np.uint32)
-            pool_d = np.full((m, pstride), np.inf, dtype=np.float32)
+            pool_ids = np.empty((m, pstride), dtype=np.uint32)
+            pool_d = np.empty((m, pstride), dtype=np.float32)
         stats = np.zeros((m, 4), dtype=np.uint32) if return_stats else None
         if m:
             check(lib().lqg_search_batch(
@@ -269,7 +272,7 @@ class Index:
                 if ef_arr.shape != (m,):
                     raise ValueError("per-query ef must have one value per query row")
                 ef0 = int(ef_arr.max()) if m else 1
-        ids = np.full((m, k), LQG_NO_ID, dtype=np.uint32)
+        ids = np.empty((m, k), dtype=np.uint32)  # every slot is written by the call
         stats = np.zeros((m, 4), dtype=np.uint32) if return_stats else None
         if m:
             check(lib().lqg_fs_search_batch(self.handle, _p(q), m, None, k, _p(ef_arr), ef0,

@@ -1,5 +1,5 @@
-// Batched-acceptance search kernel, query-per-block instances (4 warps per
-// query, 4 lanes per candidate), for small batches.
+// Batched-acceptance search kernel, latency form (one query per block: a merging
+// warp and expanding warps), for small batches.
 #include "batch_kernel.cuh"
 
 namespace lqg {
@@ -7,10 +7,10 @@ namespace lqg {
 cudaError_t launch_batch_cta(const SearchArgs& a, const ReplayArgs& ra, int degw, int blocks,
                              cudaStream_t st, int* occ) {
     switch (degw) {
-        case 1: return batch_run<1, 3>(a, ra, 1, blocks, st, occ);
-        case 2: return batch_run<2, 3>(a, ra, 1, blocks, st, occ);
-        case 3: return batch_run<3, 3>(a, ra, 1, blocks, st, occ);
-        case 4: return batch_run<4, 3>(a, ra, 1, blocks, st, occ);
+        case 1: return batch_run<1, true>(a, ra, 1, blocks, st, occ);
+        case 2: return batch_run<2, true>(a, ra, 1, blocks, st, occ);
+        case 3: return batch_run<3, true>(a, ra, 1, blocks, st, occ);
+        case 4: return batch_run<4, true>(a, ra, 1, blocks, st, occ);
         default: return cudaErrorInvalidValue;
     }
 }

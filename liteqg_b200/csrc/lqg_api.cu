@@ -291,7 +291,8 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         // the batch can be resident at once
         bool cta = false;
         if (batch && b.small_ok && t.small_batch != LQG_SMALL_BATCH_OFF &&
-            lqg::batch_smem_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap, 1) <= 227 * 1024) {
+            lqg::batch_smem_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap, 1) + 8 * ix->deg <=
+                227 * 1024) {
             if (plain) {
                 cta = true;  // one query: no occupancy question
             } else {

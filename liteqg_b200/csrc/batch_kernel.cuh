@@ -44,7 +44,7 @@
 //
 // Lazy mode (ReplayArgs::lazy) keeps no search heap while the smallest
 // unpopped distance is unique (the heap's top is then the sorted pool's first
-// unpopped entry) and rebuilds it from the logs at the first tie (below).
+// unpopped entry) and brings it up to date from the logs at a tie (below).
 //
 // A query whose search pool, sorted pool or log outgrows its capacity goes to
 // the exact global-memory kernel through the spill list.
@@ -62,18 +62,20 @@ namespace lqg {
 
 // Shared memory of one search warp: byte offsets of its parts.
 struct BatchLayout {
-    uint32_t planes, state, vis, cand, heap, pool, total;
+    uint32_t planes, state, vis, cand, heap, pool, popped, total;
 };
+constexpr uint32_t kPoppedBits = 10, kPoppedSlots = 1u << kPoppedBits;
 __host__ __device__ inline BatchLayout batch_layout(uint32_t dim, uint32_t deg, uint32_t vbits,
                                                     uint32_t scap, uint32_t acap, bool pair = false) {
     BatchLayout L;
     L.planes = 4u * ((dim + 15u) & ~15u);            // after the query
     L.state = L.planes + 2u * filter_plane(dim);     // WarpState
-    L.vis = L.state + 32u;                           // visited cache
+    L.vis = L.state + 48u;                           // visited cache
     L.cand = L.vis + (4u << vbits);                  // candidate ids, distances (pair: two)
     L.heap = L.cand + (pair ? 16u : 8u) * deg;       // search heap
     L.pool = L.heap + 8u * scap;                     // sorted pool: distances, ids
-    L.total = L.pool + 8u * acap;
+    L.popped = L.pool + 8u * acap;                   // pair: popped ids
+    L.total = L.popped + (pair ? 4u * kPoppedSlots : 0u);
     return L;
 }
 
@@ -84,8 +86,10 @@ struct WarpState {
     uint32_t qi;
     uint32_t pops, calcs;
     float smax, n2;  // the filter's per-index sums
+    uint32_t hpush, hpop;  // lazy mode: pushes and pops that the search heap holds
+    uint32_t pad[2];
 };
-static_assert(sizeof(WarpState) == 32, "BatchLayout reserves 32 bytes");
+static_assert(sizeof(WarpState) == 48, "BatchLayout reserves 48 bytes");
 
 // After a search, a warp's visited cache, candidates, search heap and sorted
 // pool (contiguous) can hold a result heap of rcap slots.
@@ -97,19 +101,22 @@ __host__ __device__ inline bool batch_replays_in_place(uint32_t deg, uint32_t vb
 
 constexpr uint32_t kPopped = 0x80000000u;  // sorted-pool id flag (ids are < 2^31)
 
-// Rebuilds the search heap of a query that ran without it (lazy mode): the
-// reference's pushes (every accepted node in order, read from the result log)
-// and pops (each after the logged number of pushes) replayed on an empty
-// heap. Every replayed pop must return the node the lazy search popped there.
-// Returns the heap's size, or kNoId (heap unusable) when one does not or the
-// heap would outgrow its slots. Not inlined: few queries come here, and the
+// The search heap of a query that runs without one (lazy mode), brought up to
+// date: the reference's pushes (every accepted node in order, read from the
+// result log) and pops (each after the logged number of pushes) since the heap
+// was last up to date (`pushed` pushes and `popped` pops, 0 and 0 at first; sn
+// entries). Every replayed pop must return the node that the lazy search popped
+// there. Returns the heap's size, or kNoId (heap unusable) when one does not or
+// the heap would outgrow its slots. Not inlined: few pops come here, and the
 // search loop has to stay in the instruction cache.
-static __device__ __noinline__ uint32_t rebuild_search_heap(const heapops::HeapView sp, uint32_t sp_max,
-                                                     const uint4* rlog, const uint2* plog,
-                                                     uint32_t acc_n, uint32_t pops, int lane) {
+static __device__ __noinline__ uint32_t update_search_heap(const heapops::HeapView sp,
+                                                           uint32_t sp_max, const uint4* rlog,
+                                                           const uint2* plog, uint32_t sn,
+                                                           uint32_t pushed, uint32_t popped,
+                                                           uint32_t acc_n, uint32_t pops, int lane) {
     using namespace heapops;
-    uint32_t sn = 0, i = 0;
-    for (uint32_t j = 0; j <= pops; ++j) {
+    uint32_t i = pushed;
+    for (uint32_t j = popped; j <= pops; ++j) {
         const uint2 pj = j < pops ? plog[j] : make_uint2(acc_n, kNoId);
         while (i < pj.x) {
             const uint32_t cnt = min(32u, pj.x - i);
@@ -199,9 +206,11 @@ constexpr uint32_t kPairRedo = 16u; // the step's expansion does not count; expa
 // messages are double-buffered. Where the next pop is not certain - equal
 // smallest distances, or the search heap in use - the expanders wait a step for
 // warp 0 to pop. The nearest candidate can be a node that the visited cache forgot and
-// that was popped before; then warp 0 finds another first entry after the
-// merge, the expansion is discarded (kPairRedo), and its marks in the visited
-// cache are true ones, since every neighbour of a popped node has been visited.
+// that was popped before. A table of the popped ids keeps most of them from being
+// expanded again (without it a third of the pops at ef 200 and degree 96 were);
+// for the rest, warp 0 finds another first entry after the merge, the expansion is
+// discarded (kPairRedo), and its marks in the visited cache are true ones, since
+// every neighbour of a popped node has been visited.
 //
 // WIDE: rows of kWideDim code bytes or more.
 //
@@ -278,12 +287,12 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
     uint32_t acc_n = 0;  // accepted so far (rp.size() = min(acc_n, ef))
     uint32_t alen = 0;   // sorted-pool entries
     float lower = INF;
-    // Lazy mode: no search heap until a pop meets a tie. The heap's live entries
-    // (distance <= lowerBound; the others are never popped) are exactly the
-    // unpopped entries of the sorted pool, so while the smallest of them is
+    // Lazy mode: no search heap except for pops that meet a tie. The heap's live
+    // entries (distance <= lowerBound; the others are never popped) are exactly
+    // the unpopped entries of the sorted pool, so while the smallest of them is
     // unique it is the heap's top. `cur` is the first unpopped entry; pops are
-    // logged (pushes are the result log) so the heap can be rebuilt when the
-    // smallest distance is shared. sn: the heap's size.
+    // logged (pushes are the result log) so the heap can be brought up to date
+    // when the smallest distance is shared. sn: the heap's size; heap: not lazy.
     bool heap = false;
     uint32_t sn = 0, cur = 0;
     uint32_t pops = 0;     // NE: pops and the query's logs (else in ws, to save registers)
@@ -299,6 +308,21 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
         if (a.esum)
 #pragma unroll
             for (int w = 0; w < DEGW; ++w) sv[w] = __ldg(a.esum + o + 32 * w);
+    };
+    // NE: the popped ids, by linear probing over 8 slots (it may miss one)
+    uint32_t* const popped = reinterpret_cast<uint32_t*>(wb + L.popped);
+    auto find_popped = [&](uint32_t id, bool insert) -> bool {
+        const uint32_t h = (id * 0x9E3779B1u) >> (32 - kPoppedBits);
+        for (uint32_t i = 0; i < 8; ++i) {
+            uint32_t* const e = popped + ((h + i) & (kPoppedSlots - 1));
+            const uint32_t was = *e;
+            if (was == id) return true;
+            if (was == kNoId) {
+                if (insert) *e = id;
+                return false;
+            }
+        }
+        return false;
     };
     auto prefetch_list = [&](uint32_t node) {
         if (lane < 2 * DEGW) {
@@ -503,16 +527,65 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
             }
             const float dn = ad[min(nxt, acap - 1)];
             if (NE > 0) tie = nn < alen && ad[nn] == dn;
+            uint32_t at = cur;  // the popped entry
             if (nxt < alen && dn == ad[cur]) {
-                // equal smallest distances: the heap layout decides
+                // equal smallest distances: the heap layout decides. The heap
+                // is brought up to date and gives this pop.
                 const size_t lo = (size_t)ws->qi * ra.rlog_cap;
-                sn = rebuild_search_heap(sp, ra.scap + ra.gcap, ra.rlog + lo, ra.plog + lo,
-                                         acc_n, NE ? pops : ws->pops, lane);
-                if (sn == kNoId) {
+                const uint32_t np = NE ? pops : ws->pops;
+                sn = update_search_heap(sp, ra.scap + ra.gcap, ra.rlog + lo, ra.plog + lo, sn,
+                                        NE ? ws->hpush : 0, NE ? ws->hpop : 0, acc_n, np, lane);
+                if (sn == kNoId || sn == 0) {
                     fail = true;
                     return false;
                 }
-                heap = true;
+                if (NE == 0) {
+                    // one warp per query: the heap is kept from here on
+                    heap = true;
+                } else {
+                    // beside expanding warps the pool's order lets them go on
+                    u = sp.get(0).x;
+                    const float d = ad[cur];
+                    __syncwarp();
+                    warp_pop(sp, sn, lane);
+                    if (lane == 0) {
+                        ws->hpush = acc_n;
+                        ws->hpop = np + 1;
+                    }
+                    // it is one of the unpopped entries at the smallest distance
+                    bool found = false;
+#pragma unroll 1
+                    for (uint32_t x0 = cur; x0 < alen && !found; x0 += 32) {
+                        const uint32_t x = x0 + lane;
+                        const unsigned hit =
+                            __ballot_sync(kFull, x < alen && ad[x] == d && ai[x] == u);
+                        if (hit) {
+                            at = x0 + __ffs(hit) - 1;
+                            found = true;
+                        } else if (ad[min(x0 + 31, alen - 1)] != d) {
+                            break;
+                        }
+                    }
+                    if (!found) {
+                        fail = true;
+                        return false;
+                    }
+                }
+            }
+            if (NE > 0 || !heap) {
+                __syncwarp();
+                if (lane == 0) {
+                    ai[at] = u | kPopped;
+                    // (pops < accepted nodes <= rlog_cap)
+                    if (NE)
+                        plg[pops] = make_uint2(acc_n, u);
+                    else
+                        ra.plog[(size_t)ws->qi * ra.rlog_cap + ws->pops] = make_uint2(acc_n, u);
+                }
+                if (at == cur)
+                    cur = nxt;
+                else if (NE > 0)
+                    tie = nxt == at ? nn < alen && ad[nn] == ad[cur] : true;
             }
         }
         if (heap) {
@@ -521,17 +594,6 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
             if (-__uint_as_float(top.y) > lower) return false;
             warp_pop(sp, sn, lane);
             u = top.x;
-        } else {
-            __syncwarp();
-            if (lane == 0) {
-                ai[cur] = u | kPopped;
-                // (pops < accepted nodes <= rlog_cap)
-                if (NE)
-                    plg[pops] = make_uint2(acc_n, u);
-                else
-                    ra.plog[(size_t)ws->qi * ra.rlog_cap + ws->pops] = make_uint2(acc_n, u);
-            }
-            cur = nxt;
         }
         if (NE)
             ++pops;
@@ -631,6 +693,9 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
 #pragma unroll 1
             for (uint32_t i = 4 * lane; i < (1u << vbits); i += 128)
                 *reinterpret_cast<uint4*>(vis.s + 2 * i) = make_uint4(0, 0, 0, 0);
+            if (NE)
+                for (uint32_t i = 4 * lane; i < kPoppedSlots; i += 128)
+                    *reinterpret_cast<uint4*>(popped + i) = make_uint4(kNoId, kNoId, kNoId, kNoId);
             __syncwarp();
             const Sq8Filter f =
                 filter_prepare(qs, pmin, pscale, dim, ws->smax, ws->n2, planes, lane);
@@ -641,6 +706,7 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
                 ws->qi = qi;
                 ws->pops = 0;
                 ws->calcs = 1;
+                ws->hpush = ws->hpop = 0;
                 // qg.hpp:305-311: the entry point seeds both pools and is
                 // visited; here it is the first round's only candidate
                 cand[0] = a.entry;
@@ -731,6 +797,7 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
                         uint32_t total = 0;
                         if (hw == 1) {
                             load_list(x);
+                            if (lane == 0) find_popped(x, true);
                             total = expand(cn, cd);
                         }
                         uint32_t s0 = 0;
@@ -747,7 +814,9 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
                         n = measure(cn + s0, cd + s0, n, flags & kPairFull, bound);
                         for (uint32_t c0 = 0; c0 < n; c0 += 32) {
                             const uint32_t c = c0 + lane;
-                            const uint32_t yb = c < n ? __float_as_uint(cd[s0 + c]) : 0xFFFFFFFFu;
+                            const uint32_t yb = c < n && !find_popped(cn[s0 + c], false)
+                                                    ? __float_as_uint(cd[s0 + c])
+                                                    : 0xFFFFFFFFu;
                             const uint32_t m = __reduce_min_sync(kFull, yb);
                             const unsigned at = __ballot_sync(kFull, yb == m);
                             if (m == mb) ++same;

@@ -197,6 +197,14 @@ lqg_status reset_ctl(Workspace& w, cudaStream_t st) {
     return LQG_OK;
 }
 
+// The tuned visited-cache bits, or what names the index's ids uniquely
+// (VisitedCache) if that is more.
+uint32_t least_visited_bits(const lqg_index* ix) {
+    uint32_t vb = ix->tune.visited_bits;
+    while (vb < 15 && ix->n > (1ull << (vb + 16))) ++vb;
+    return vb;
+}
+
 // Visited-cache bits of a batch-kernel launch of m queries, `warps` per block.
 // A larger cache forgets fewer nodes (at ef 200 and degree 96: 10.5 k
 // evaluations per query at 10 bits, 6.5 k at 13, 5.6 k without forgetting), but
@@ -204,10 +212,9 @@ lqg_status reset_ctl(Workspace& w, cudaStream_t st) {
 // (1M x 128, 10,000 queries at ef 64: 2.75 ms at 10, 2.95 at 11, 4.45 at 12).
 // So a batch whose queries all fit at once takes the largest cache they fit
 // with, when the tuning field is at its default; other values are taken as they
-// are. Ids of the index must name slot and tag uniquely (batch_kernel.cuh).
+// are.
 uint32_t batch_visited_bits(const lqg_index* ix, const lqg::ReplayArgs& ra, int64_t m, int warps) {
-    uint32_t vb = ix->tune.visited_bits;
-    while (vb < 15 && ix->n > (1ull << (vb + 16))) ++vb;
+    const uint32_t vb = least_visited_bits(ix);
     if (vb != 10) return vb;
     for (uint32_t x = 13; x > vb; --x) {
         const size_t smem = lqg::batch_smem_bytes(ix->dim, ix->deg, x, ra.scap, ra.acap, warps);
@@ -215,6 +222,30 @@ uint32_t batch_visited_bits(const lqg_index* ix, const lqg::ReplayArgs& ra, int6
         if (smem <= 227 * 1024 && per_sm * warps * ix->num_sms >= m) return x;
     }
     return vb;
+}
+
+// The same for the latency form with nb blocks per SM, where shared memory is
+// plentiful: first room for the search heap of a query that meets a tie (past
+// its slots in shared memory a push waits for global memory: one tie cost a
+// query of 560 us another 350 at 256 slots), then the largest visited cache, up
+// to 2^14 (clearing it costs about 600 cycles per query).
+void latency_shape(const lqg_index* ix, int nb, uint32_t& vbits, lqg::ReplayArgs& ra) {
+    const size_t budget = std::min<size_t>(227 * 1024, 228 * 1024 / nb - 1024);
+    auto fits = [&](uint32_t vb, uint32_t scap) {
+        return lqg::batch_latency_bytes(ix->dim, ix->deg, vb, scap, ra.acap) <= budget;
+    };
+    if (ix->tune.heap_scap == 256)
+        for (uint32_t c = 2048; c > 256; c /= 2)
+            if (fits(vbits, c)) {
+                ra.scap = c;
+                break;
+            }
+    if (ix->tune.visited_bits == 10)
+        for (uint32_t x = 14; x > vbits; --x)
+            if (fits(x, ra.scap)) {
+                vbits = x;
+                break;
+            }
 }
 
 // Fast kernel over all queries, then the exact kernel over the flagged ones.
@@ -286,13 +317,13 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         ra.swarps = (uint32_t)sw;
         SearchArgs h = base_args(ix, w, b);
         h.qhead = w.d_ctl + kCtlHeapHead;
-        h.vbits = batch ? batch_visited_bits(ix, ra, b.m, sw) : t.visited_bits;
-        // small batches: one query per block of 4 warps, when every query of
-        // the batch can be resident at once
+        h.vbits = batch ? least_visited_bits(ix) : t.visited_bits;
+        // small batches: the latency form, when every query of the batch can be
+        // resident at once
         bool cta = false;
         if (batch && b.small_ok && t.small_batch != LQG_SMALL_BATCH_OFF &&
-            lqg::batch_smem_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap, 1) + 8 * ix->deg <=
-                227 * 1024) {
+            lqg::batch_latency_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap) <= 227 * 1024) {
+            int nb = 1;  // blocks per SM
             if (plain) {
                 cta = true;  // one query: no occupancy question
             } else {
@@ -303,8 +334,11 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
                                         ? (int64_t)oc * ix->num_sms
                                         : t.small_batch;
                 cta = oc > 0 && b.m <= lim;
+                nb = (int)std::min<int64_t>(oc, (b.m + ix->num_sms - 1) / ix->num_sms);
             }
+            if (cta) latency_shape(ix, nb, h.vbits, ra);
         }
+        if (batch && !cta) h.vbits = batch_visited_bits(ix, ra, b.m, sw);
         if (cta) sw = 1;
         // the batch kernels' distance passes use 4 lanes per candidate; the
         // tuning field keeps its accepted values

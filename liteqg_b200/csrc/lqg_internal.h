@@ -88,13 +88,15 @@ cudaError_t launch_split(const SearchArgs& a, const ReplayArgs& ra, int E, int G
 // sorted pool in shared memory, each expansion's candidates decided at once.
 size_t batch_smem_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t scap, uint32_t acap,
                         int warps);
+// ... of a block of the latency form
+size_t batch_latency_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t scap, uint32_t acap);
 bool batch_replays_in_place_host(uint32_t deg, uint32_t vbits, uint32_t scap, uint32_t acap,
                                  uint32_t rcap);
 cudaError_t launch_batch(const SearchArgs& a, const ReplayArgs& ra, int degw, int warps, int blocks,
                          cudaStream_t st, int* occ);
-// Its query-per-block form (batch_cta.cu): one query per block of 4 warps,
-// each expansion's distances split over the warps; for batches smaller than
-// the GPU's resident warps, where a query's latency sets the batch time.
+// Its latency form (batch_cta.cu): one query per block of a merging warp and
+// one or three expanding warps; for batches whose queries all fit on the GPU at
+// once, where a query's latency sets the batch time.
 cudaError_t launch_batch_cta(const SearchArgs& a, const ReplayArgs& ra, int degw, int blocks,
                              cudaStream_t st, int* occ);
 // Result-heap replay pass over a[0, m): one warp per query.

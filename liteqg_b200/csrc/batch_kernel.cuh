@@ -141,7 +141,7 @@ static __device__ __noinline__ uint32_t update_search_heap(const heapops::HeapVi
 // __grid_constant__ kernel parameters: nothing is copied.)
 static __device__ __noinline__ bool replay_result_call(const SearchArgs& a, const ReplayArgs& ra,
                                                        int64_t qi, uint32_t len,
-                                                       const heapops::HeapView rp, int lane) {
+                                                       const heapops::SharedHeap rp, int lane) {
     return replay_result(a, ra, qi, len, rp, lane);
 }
 
@@ -906,7 +906,7 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
         if (!fail && !direct && !ra.replay_all &&
             batch_replays_in_place(32 * DEGW, vbits, ra.scap, acap, ra.rcap)) {
             __syncwarp();
-            const HeapView rph{reinterpret_cast<uint2*>(wb + L.vis), nullptr, ra.rcap};
+            const SharedHeap rph(wb + L.vis);
             fail = !replay_result_call(a, ra, qi, acc_n, rph, lane);
             direct = !fail;
         }

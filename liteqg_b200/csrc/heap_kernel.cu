@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256, 2) heap_search_kernel(SearchArgs a, HeapA
     uint32_t* cid = vis + vsize;
     float* cd = reinterpret_cast<float*>(cid + kMaxDeg);
     uint2* rps = reinterpret_cast<uint2*>(cd + kMaxDeg);
-    const HeapView rp{rps, nullptr, hp.rcap};
+    const SharedHeap rp(rps);
     const size_t gw = (size_t)blockIdx.x * (blockDim.x >> 5) + warp;
     const HeapView sp{rps + hp.rcap, hp.sp_global + gw * hp.gcap, hp.scap};
     const uint32_t sp_max = hp.scap + hp.gcap;

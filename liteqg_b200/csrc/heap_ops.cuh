@@ -1,16 +1,12 @@
 // Warp-cooperative libstdc++ binary-heap steps on (id, distance bits) pairs,
-// shared by the heap and split search kernels. comp(x, y) is x.dist < y.dist
+// shared by the search kernels that keep heaps. comp(x, y) is x.dist < y.dist
 // (symqglib/qg/qg.hpp:289-293); the search pool stores -distance.
 //   push: sift-up while comp(parent, value) (GCC bits/stl_heap.h
-//         __push_heap). The path from the new slot to the root is known and
-//         comp(parent, value) is monotone along it, so lane i loads the i-th
-//         ancestor, one ballot gives how far the value rises, and the shifted
-//         ancestors are written in one step.
+//         __push_heap).
 //   pop:  move the last element out, walk a hole from the root to a leaf
 //         along the larger child (the right one unless comp(right, left)),
 //         then sift the moved element up from there (__pop_heap /
-//         __adjust_heap). The walk is data dependent and runs on lane 0; the
-//         sift-up is the warp-parallel one.
+//         __adjust_heap).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -25,100 +21,154 @@ __device__ __forceinline__ bool hless(uint2 x, uint2 y) {
     return __uint_as_float(x.y) < __uint_as_float(y.y);
 }
 
+// A heap array wholly in shared memory, by its address there: in a function that
+// is not inlined a pointer would make every access a generic one.
+struct SharedHeap {
+    uint32_t s;
+    __device__ __forceinline__ explicit SharedHeap(const void* p)
+        : s((uint32_t)__cvta_generic_to_shared(p)) {}
+    __device__ __forceinline__ uint2 get(uint32_t i) const {
+        uint2 v;
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];"
+                     : "=r"(v.x), "=r"(v.y)
+                     : "r"(s + 8 * i)
+                     : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void set(uint32_t i, uint2 v) const {
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(s + 8 * i), "r"(v.x), "r"(v.y)
+                     : "memory");
+    }
+};
+
 // A heap array: slots [0, cap) in shared memory, slots >= cap (the deepest
 // levels of a large search pool) in a per-warp global-memory area.
 struct HeapView {
-    uint2* s;
+    SharedHeap s;
     uint2* g;
     uint32_t cap;
-    __device__ __forceinline__ uint2 get(uint32_t i) const { return i < cap ? s[i] : g[i - cap]; }
+    __device__ __forceinline__ HeapView(uint2* smem, uint2* global, uint32_t slots)
+        : s(smem), g(global), cap(slots) {}
+    __device__ __forceinline__ uint2 get(uint32_t i) const {
+        return i < cap ? s.get(i) : g[i - cap];
+    }
     __device__ __forceinline__ void set(uint32_t i, uint2 v) const {
         if (i < cap)
-            s[i] = v;
+            s.set(i, v);
         else
             g[i - cap] = v;
     }
 };
 
-// Sift-up of v from slot `hole` (libstdc++ __push_heap with top 0), all lanes.
-__device__ __forceinline__ void warp_sift_up(HeapView h, uint32_t hole, uint2 v, int lane) {
-    // ancestors of hole: ((hole + 1) >> i) - 1 for i = 1 .. depth
-    const uint32_t p1 = hole + 1;
-    const uint32_t depth = 31u - __clz(p1);  // floor(log2(hole + 1))
-    bool pred = false;
-    uint2 anc = make_uint2(0, 0);
-    if (lane >= 1 && (uint32_t)lane <= depth) {
-        anc = h.get((p1 >> lane) - 1u);
-        pred = hless(anc, v);
+// push_heap of v at slot n, all lanes: lane i takes the i-th ancestor of the new
+// slot, ((n + 1) >> i) - 1. The value rises past the ancestors up to the first
+// that is not less than it; each lane reads off one ballot whether it is among
+// them, so the moves need no further exchange.
+template <class H>
+__device__ __forceinline__ void push_steps(H h, uint32_t& n, uint2 v, int lane) {
+    const uint32_t p1 = n + 1;
+    const uint32_t a = p1 >> lane;
+    bool less = false;
+    uint2 anc = v;
+    if (lane > 0 && a > 0) {
+        anc = h.get(a - 1);
+        less = hless(anc, v);
     }
-    const unsigned m = __ballot_sync(kFull, pred);
-    // consecutive trues from level 1 upward: the loop of __push_heap stops
-    // at the first parent that is not less than the value
-    const uint32_t j = (uint32_t)(__ffs(~(m >> 1)) - 1);
-    // level l (1..j): its value moves down to level l - 1
-    if (lane >= 1 && (uint32_t)lane <= j) h.set((p1 >> (lane - 1)) - 1u, anc);
-    if (lane == 0) h.set((p1 >> j) - 1u, v);
+    const unsigned m = __ballot_sync(kFull, less) | 1u;  // (lane 0: the new slot)
+    const unsigned upto = (2u << lane) - 1u;
+    if ((m & upto) == upto) {  // v passes this level
+        if (lane > 0) h.set((p1 >> (lane - 1)) - 1u, anc);
+        if (((m >> lane) >> 1 & 1u) == 0) h.set(a - 1, v);  // and stays here
+    }
     __syncwarp();
-}
-
-__device__ __forceinline__ void warp_push(HeapView h, uint32_t& n, uint2 v, int lane) {
-    warp_sift_up(h, n, v, lane);
     ++n;
 }
 
-// pop_heap + pop_back. The hole walk of __adjust_heap goes five levels per
+// A heap that so far lies in shared memory takes the steps without the choice of
+// memory in each access (a push of 350 cycles takes 257).
+template <class H>
+__device__ __forceinline__ void warp_push(H h, uint32_t& n, uint2 v, int lane) {
+    push_steps(h, n, v, lane);
+}
+__device__ __forceinline__ void warp_push(HeapView h, uint32_t& n, uint2 v, int lane) {
+    if (n < h.cap)
+        push_steps(h.s, n, v, lane);
+    else
+        push_steps(h, n, v, lane);
+}
+
+// pop_heap + pop_back. __adjust_heap moves the larger child up into the hole as
+// far as a leaf, and __push_heap then lifts the last element v from there past
+// the moved values that are less than v. These do not increase along the path,
+// so v ends where the first of them is less than it, and the values below that
+// slot are back where they were: the walk stops there. It goes five levels per
 // round: lane i (< 31) takes the i-th node, in breadth-first order, of the
-// five-level subtree under the hole, loads its two children and decides
-// which one the walk would take from it (left only if comp(right, left)) and
-// whether the walk continues there (node < (len - 1) / 2). One ballot per
-// bit gives the path; each lane on it moves its chosen child up into its
-// node. All loads of a round precede its stores and no path node is read
+// five-level subtree under the hole, loads its children and decides which one
+// the walk would take (left only if comp(right, left), or alone) and whether
+// the walk goes on (v does not stay). Two ballots tell each lane whether it is on
+// the path. All loads of a round precede its stores and no path node is read
 // after it is written, so the moves are the sequential walk's.
-__device__ __forceinline__ void warp_pop(HeapView h, uint32_t& n, int lane) {
+// (A lone warp, 256 entries: 729 cycles, 1,012 with the walk to the leaf and back
+// on the ballots' bits; a push 225, it took 378.)
+template <class H>
+__device__ __forceinline__ void pop_steps(H h, uint32_t& n, int lane) {
     const uint32_t size = n;
     if (size > 1) {
         const uint32_t len = size - 1;
         const uint2 v = h.get(len);
-        const uint32_t lim = (len - 1) / 2;
+        // breadth-first index i: depth k = floor(log2(i + 1)), offset i + 1 - 2^k;
+        // anc: its ancestors' bits, lefts: those it lies to the left of
+        const uint32_t i1 = (uint32_t)lane + 1u;
+        const uint32_t k = 31u - __clz(i1);
+        const uint32_t off = i1 - (1u << k);
+        unsigned anc = 0, lefts = 0;
+#pragma unroll
+        for (int t = 1; t <= 4; ++t) {
+            const unsigned bit = (1u << (i1 >> t)) >> 1;  // 0 above the root
+            anc |= bit;
+            if (((i1 >> (t - 1)) & 1u) == 0) lefts |= bit;
+        }
         uint32_t hole = 0;
-        // BFS index i: depth k = floor(log2(i + 1)), offset i + 1 - 2^k
-        const uint32_t k = 31u - __clz((uint32_t)lane + 1u);
-        const uint32_t off = (uint32_t)lane + 1u - (1u << k);
-        while (hole < lim) {
+        while (true) {
             const uint32_t node = ((hole + 1u) << k) - 1u + off;
-            const bool cont = lane < 31 && node < lim;
-            uint2 ch = make_uint2(0, 0);
-            bool left = false;
-            if (cont) {
-                const uint2 r = h.get(2 * node + 2), l = h.get(2 * node + 1);
-                left = hless(r, l);
-                ch = left ? l : r;
+            const uint32_t c = 2 * node + 1;
+            bool go = false, left = true;
+            uint2 ch = v;
+            if (lane < 31 && c < len) {
+                const uint2 l = h.get(c);
+                ch = l;
+                if (c + 1 < len) {
+                    const uint2 r = h.get(c + 1);
+                    left = hless(r, l);
+                    ch = left ? l : r;
+                }
+                go = !hless(ch, v);
             }
-            const unsigned mc = __ballot_sync(kFull, cont);
+            const unsigned mg = __ballot_sync(kFull, go);
             const unsigned ml = __ballot_sync(kFull, left);
-            uint32_t i = 0, path = 0;
-            int steps = 0;
-            while (steps < 5 && ((mc >> i) & 1u)) {
-                path |= 1u << i;
-                i = 2 * i + (((ml >> i) & 1u) ? 1u : 2u);
-                ++steps;
-            }
-            if ((path >> lane) & 1u) h.set(node, ch);
-            __syncwarp();
-            // the hole moves to BFS index i (depth `steps`) of this subtree
-            hole = ((hole + 1u) << steps) - 1u + (i + 1u - (1u << steps));
-            if (steps < 5) break;
+            const bool move = go && (mg & anc) == anc && (ml & anc) == lefts;
+            if (move) h.set(node, ch);
+            const unsigned mv = __ballot_sync(kFull, move);
+            if (mv == 0) break;
+            const int last = 31 - __clz(mv);  // the deepest
+            hole = __shfl_sync(kFull, left ? c : c + 1, last);
+            if (last < 15) break;  // above the fifth level
         }
-        if ((len & 1u) == 0 && hole == (len - 2) / 2) {
-            const uint2 c = h.get(2 * hole + 1);
-            __syncwarp();
-            if (lane == 0) h.set(hole, c);
-            __syncwarp();
-            hole = 2 * hole + 1;
-        }
-        warp_sift_up(h, hole, v, lane);
+        if (lane == 0) h.set(hole, v);
+        __syncwarp();
     }
     n = size - 1;
+}
+
+template <class H>
+__device__ __forceinline__ void warp_pop(H h, uint32_t& n, int lane) {
+    pop_steps(h, n, lane);
+}
+__device__ __forceinline__ void warp_pop(HeapView h, uint32_t& n, int lane) {
+    if (n <= h.cap)
+        pop_steps(h.s, n, lane);
+    else
+        pop_steps(h, n, lane);
 }
 
 }  // namespace heapops
@@ -131,14 +181,14 @@ __device__ __forceinline__ void warp_pop(HeapView h, uint32_t& n, int lane) {
 // in ascending order. The log is read 32 entries per coalesced load. Returns
 // false (nothing written) when a check fails.
 __device__ __forceinline__ bool replay_result(const SearchArgs& a, const ReplayArgs& ra,
-                                              int64_t qi, uint32_t len, const heapops::HeapView rp,
+                                              int64_t qi, uint32_t len, const heapops::SharedHeap rp,
                                               int lane) {
     using namespace heapops;
     const uint32_t efq = query_ef(a, qi);
     const uint32_t ef = min(max(efq, 1u), ra.efcap);
     const uint32_t k = min(a.kq ? a.kq[qi] : a.k0, a.kstride);
     const uint4* lg = ra.rlog + (size_t)qi * ra.rlog_cap;
-    uint32_t n = 0;
+    uint32_t n = 0, top = 0;
     bool ok = len > 0 && len <= ra.rlog_cap;
     for (uint32_t b = 0; ok && b < len; b += 32) {
         const uint4 mine = b + lane < len ? __ldcs(lg + b + lane) : make_uint4(0, 0, 0, 0);
@@ -147,13 +197,14 @@ __device__ __forceinline__ bool replay_result(const SearchArgs& a, const ReplayA
             const uint32_t id = __shfl_sync(kFull, mine.x, j);
             const uint32_t yb = __shfl_sync(kFull, mine.y, j);
             const uint32_t lb = __shfl_sync(kFull, mine.z, j);
-            if (!(n < ef || __uint_as_float(rp.get(0).y) > __uint_as_float(yb))) {
+            if (!(n < ef || __uint_as_float(top) > __uint_as_float(yb))) {
                 ok = false;
                 break;
             }
             warp_push(rp, n, make_uint2(id, yb), lane);
             if (n > ef) warp_pop(rp, n, lane);
-            if (rp.get(0).y != lb) {
+            top = rp.get(0).y;
+            if (top != lb) {
                 ok = false;
                 break;
             }

@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) rp_replay_kernel(SearchArgs a, ReplayArgs
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
-    const HeapView rp{hs + (size_t)warp * ra.rcap, nullptr, ra.rcap};
+    const SharedHeap rp(hs + (size_t)warp * ra.rcap);
     for (int64_t qi = (int64_t)blockIdx.x * wpb + warp; qi < a.m; qi += (int64_t)gridDim.x * wpb) {
         const uint32_t len = ra.rlen[qi];
         // kNoId: the search failed (already on the spill list); kRlenDone: the

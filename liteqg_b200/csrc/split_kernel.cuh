@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(160, 4) split_search_kernel(SearchArgs a, Repl
         // free now), else in the result replay pass
         if (!fail && !direct && !ra.replay_all && split_replays_in_place(vbits, ra.scap, ra.rcap)) {
             __syncwarp();
-            const HeapView rph{reinterpret_cast<uint2*>(vis), nullptr, ra.rcap};
+            const SharedHeap rph(vis);
             fail = !replay_result(a, ra, qi, acc_n, rph, lane);
             direct = !fail;
         }

@@ -197,6 +197,10 @@ lqg_status reset_ctl(Workspace& w, cudaStream_t st) {
     return LQG_OK;
 }
 
+// The tuned search-heap slots, an even number: warps' areas follow each other in
+// shared memory, and their queries are read 16 bytes at a time.
+uint32_t heap_slots(const lqg_tuning& t) { return (t.heap_scap + 1u) & ~1u; }
+
 // The tuned visited-cache bits, or what names the index's ids uniquely
 // (VisitedCache) if that is more.
 uint32_t least_visited_bits(const lqg_index* ix) {
@@ -279,7 +283,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         lqg::ReplayArgs ra{};
         ra.rcap = (b.ef0 + 2u) & ~1u;
         ra.efcap = std::min(32u * (uint32_t)RE - 32u, ra.rcap - 1u);
-        ra.scap = t.heap_scap;
+        ra.scap = heap_slots(t);
         ra.spill = w.d_spill;
         ra.nspill = w.d_ctl + kCtlSpilled;
         ra.rlog_cap = std::max(1024u, 16u * b.ef0);
@@ -482,7 +486,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         h.vbits = t.visited_bits;
         lqg::HeapArgs hp{};
         hp.rcap = (b.ef0 + 2u) & ~1u;
-        hp.scap = t.heap_scap;
+        hp.scap = heap_slots(t);
         hp.spill = w.d_spill;
         hp.nspill = w.d_ctl + kCtlSpilled;
         int hw = plain ? 1 : (int)t.heap_warps;

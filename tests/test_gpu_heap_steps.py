@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("mode", [2, 4, 5, 6])
-@pytest.mark.parametrize("scap", [256, 1024])
+@pytest.mark.parametrize("scap", [256, 257, 1024])
 @pytest.mark.parametrize("ef", [1, 2, 3, 31, 32, 33, 62, 63, 64, 511, 512])
 def test_ties_at_the_edges_of_levels(ef, scap, mode):
     import liteqg_b200

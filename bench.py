@@ -1078,7 +1078,7 @@ def uneven_arm(args, w, name, device):
 
     best = None
     # (mode, lanes per candidate, heap warps per block, heap slots, visited
-    # bits[, 1: batch kernels one query per block of 4 warps])
+    # bits[, 1: batch kernels one query per block])
     shapes = ((6, 2, 4, 512, 10), (6, 4, 4, 512, 10), (5, 2, 4, 512, 10), (4, 4, 4, 512, 10),
               (2, 2, 4, 512, 10), (2, 4, 4, 512, 10), (1, 4, 4, 512, 10),
               (2, 2, 4, 256, 10), (2, 2, 4, 256, 9), (2, 2, 2, 512, 10), (2, 2, 8, 256, 9),
@@ -1086,7 +1086,7 @@ def uneven_arm(args, w, name, device):
               # ef up to 512, against fewer resident warps
               (2, 2, 2, 512, 12), (2, 2, 4, 256, 11), (2, 2, 2, 256, 13), (2, 2, 3, 512, 12),
               # the query-per-block form on the whole batch: 960-byte rows make
-              # the distances most of a pop, which its 4 warps share
+              # the distances most of a pop, which its warps share
               (6, 4, 4, 512, 10, 1), (6, 4, 4, 512, 11, 1), (6, 4, 4, 512, 12, 1),
               (5, 4, 4, 512, 11, 1))
     from liteqg_b200._capi import SMALL_BATCH_AUTO, LqgError
@@ -1229,7 +1229,7 @@ def uneven_arm(args, w, name, device):
                                 2: "heap_search_kernel", 4: "split_search_kernel",
                                 5: "batch_search_kernel",
                                 6: "batch_search_kernel (lazy search heap)"}.get(best[1]) +
-                               (", one query per block of 4 warps" if best[6] else "")},
+                               (", one query per block" if best[6] else "")},
         "e2e": {"value": e2e_qps, "unit": "queries/s",
                 "h2d_bytes_per_step": int(nq * dim * 4 + 8 * nq),
                 "d2h_bytes_per_step": int(nq * kmax * 4), "ids_equal": e2e_ok},

@@ -236,20 +236,23 @@ LQG_API lqg_status lqg_search_exact_noalloc(lqg_index* ix, const float* queries,
  *   heap_warps      {1..8}: warps per block of the heap kernel, {1..5} of
  *                   the split and batch kernels (modes 4-6)
  *   heap_scap       [256, 16384]: search-pool slots per query in shared
- *                   memory (heap and replay kernels; larger pools spill to
- *                   global memory, then to the global-memory kernel)
+ *                   memory (modes 2-6; larger pools spill to global memory,
+ *                   then to the global-memory kernel). At the default of 256
+ *                   the latency form takes up to 2048 where they are free
  *   replay_warps    {1..15}: search warps per block of the replay kernel
  *                   (plus one replay warp)
  *   replay_all      modes 4-6: 1 sends every query through the checked result
  *                   replay pass (0, the default: only queries whose output
  *                   the heap layout decides); set on every call, not kept
  *                   when 0 is passed
- *   small_batch     modes 5-6: a batch of at most this many queries runs one
- *                   query per block of 4 warps (each expansion's distances
- *                   split over the warps: lower latency per query, fewer
- *                   queries resident); LQG_SMALL_BATCH_AUTO (the default):
- *                   as many queries as such blocks fit on the GPU at once;
- *                   LQG_SMALL_BATCH_OFF: never. The same ids either way. */
+ *   small_batch     modes 5-6: a batch of at most this many queries runs in the
+ *                   latency form, one query per block of one merging warp and
+ *                   one or three expanding warps (lower latency per query,
+ *                   fewer queries resident); LQG_SMALL_BATCH_AUTO (the
+ *                   default): as many queries as such blocks fit on the GPU
+ *                   at once, and larger batches with per-query ef in which few
+ *                   queries have a large one; LQG_SMALL_BATCH_OFF: never. The
+ *                   same ids either way. */
 typedef struct {
     uint32_t lanes_per_cand;
     uint32_t visited_bits;

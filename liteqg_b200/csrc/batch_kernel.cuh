@@ -259,6 +259,7 @@ __global__ void __maxnreg__(WIDE || NE ? 128 : 96)
     const HeapView sp{reinterpret_cast<uint2*>(wb + L.heap), ra.sp_global + (size_t)gw * ra.gcap,
                       ra.scap};
 
+    if (a.nlist && *a.nlist == 0) return;  // the batch went to the other form
     for (uint32_t i = threadIdx.x; i < dpad; i += blockDim.x) {
         pmin[i] = i < dim ? a.params[2 * i] : 0.f;
         pscale[i] = i < dim ? a.params[2 * i + 1] : 0.f;

@@ -325,6 +325,12 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         // small batches: the latency form, when every query of the batch can be
         // resident at once
         bool cta = false;
+        // resident blocks of the latency form, if a device-side look at the
+        // queries' ef shall choose between the forms (choose_form_kernel; past 16
+        // per block it would hardly choose this one)
+        int64_t lblocks = 0;
+        SearchArgs hl{};
+        lqg::ReplayArgs rl{};
         if (batch && b.small_ok && t.small_batch != LQG_SMALL_BATCH_OFF &&
             lqg::batch_latency_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap) <= 227 * 1024) {
             int nb = 1;  // blocks per SM
@@ -339,6 +345,12 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
                                         : t.small_batch;
                 cta = oc > 0 && b.m <= lim;
                 nb = (int)std::min<int64_t>(oc, (b.m + ix->num_sms - 1) / ix->num_sms);
+                if (!cta && b.efq && t.small_batch == LQG_SMALL_BATCH_AUTO && b.m <= 16 * lim) {
+                    lblocks = lim;
+                    hl = h;
+                    rl = ra;
+                    latency_shape(ix, oc, hl.vbits, rl);
+                }
             }
             if (cta) latency_shape(ix, nb, h.vbits, ra);
         }
@@ -368,8 +380,9 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         // longest-expected queries first, when a chunk holds more queries
         // than the launch has warps (otherwise they all start at once)
         const bool order = !plain && chunk > (int64_t)rb * sw;
-        if (order && (s = ensure_order(w, chunk)) != LQG_OK) return s;
-        const size_t slots = (size_t)rb * sw;
+        // (a later batch with per-query ef may need a work list)
+        if ((order || (batch && b.efq)) && (s = ensure_order(w, chunk)) != LQG_OK) return s;
+        const size_t slots = std::max((size_t)rb * sw, (size_t)lblocks);
         if (w.sp_global_slots < slots) {
             dfree(w.d_sp_global);
             w.sp_global_slots = 0;
@@ -379,14 +392,15 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
             }
             w.sp_global_slots = slots;
         }
-        ra.sp_global = w.d_sp_global;
+        rl.sp_global = ra.sp_global = w.d_sp_global;
+        rl.gcap = kHeapGlobalCap;
         ra.gcap = kHeapGlobalCap;
         if (ix->ev_start) LQG_CUDA(cudaEventRecord(ix->ev_start, b.st));
         for (int64_t off = 0; off < b.m; off += chunk) {
             const int64_t mc = std::min(chunk, b.m - off);
             if (off > 0) {  // fresh work-queue heads and spill list for this chunk
                 LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlExactHead, 0, sizeof(uint32_t), b.st));
-                LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlHeapHead, 0, 2 * sizeof(uint32_t), b.st));
+                LQG_CUDA(cudaMemsetAsync(w.d_ctl + kCtlHeapHead, 0, 3 * sizeof(uint32_t), b.st));
             }
             SearchArgs c = h;
             c.queries += off * ix->dim;
@@ -403,6 +417,20 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
                 (s = order_queries(ix, w, c.queries, c.efq, mc, b.st, &c.qlist)) != LQG_OK)
                 return s;
             const int cb = (int)std::min<int64_t>(rb, (mc + sw - 1) / sw);
+            if (lblocks > 0) {
+                const int32_t* warp_list = c.qlist;
+                if ((s = choose_form(w, c.efq, mc, b.ef0, lblocks, b.st, &c.qlist)) != LQG_OK)
+                    return s;
+                c.nlist = w.d_ctl + kCtlLatencyCount;
+                c.qhead = w.d_ctl + kCtlLatencyHead;
+                c.vbits = hl.vbits;
+                e = lqg::launch_batch_cta(c, rl, degw, (int)std::min(lblocks, mc), b.st, nullptr);
+                if (e != cudaSuccess) return cuda_fail(e, "search launch");
+                c.qlist = warp_list;
+                c.nlist = w.d_ctl + kCtlWarpCount;
+                c.qhead = h.qhead;
+                c.vbits = h.vbits;
+            }
             e = launch(c, cb, nullptr);
             if (e != cudaSuccess) return cuda_fail(e, "search launch");
             const bool in_place =

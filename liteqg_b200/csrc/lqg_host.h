@@ -40,7 +40,11 @@ enum : int {
     kCtlErr = 3,
     kCtlErrQuery = 4,
     kCtlHeapHead = 5,
-    kCtlSpilled = 6
+    kCtlSpilled = 6,
+    kCtlLatencyHead = 7,
+    // lengths of the batch kernel's two work lists (it has no fast pass)
+    kCtlWarpCount = kCtlFastHead,
+    kCtlLatencyCount = kCtlFlagged
 };
 constexpr int kCtlWords = 8;
 
@@ -292,6 +296,8 @@ lqg_status filter_edge_sums(lqg_index* ix, cudaStream_t st);
 // Work order of a batch (order.cu): largest ef, then farthest from the entry
 // point, first.
 lqg_status ensure_order(Workspace& w, int64_t chunk);
+lqg_status choose_form(Workspace& w, const uint32_t* efq, int64_t m, uint32_t efmax,
+                       int64_t blocks, cudaStream_t st, const int32_t** list);
 lqg_status order_queries(const lqg_index* ix, Workspace& w, const float* queries,
                          const uint32_t* efq, int64_t m, cudaStream_t st, const int32_t** list);
 lqg_status search_host(lqg_index* ix, Workspace& w, const float* queries, int64_t m,

@@ -238,7 +238,8 @@ LQG_API lqg_status lqg_search_exact_noalloc(lqg_index* ix, const float* queries,
  *   heap_scap       [256, 16384]: search-pool slots per query in shared
  *                   memory (modes 2-6; larger pools spill to global memory,
  *                   then to the global-memory kernel). At the default of 256
- *                   the latency form takes up to 2048 where they are free
+ *                   modes 5-6 take 384, and in the latency form up to 2048,
+ *                   where they are free
  *   replay_warps    {1..15}: search warps per block of the replay kernel
  *                   (plus one replay warp)
  *   replay_all      modes 4-6: 1 sends every query through the checked result

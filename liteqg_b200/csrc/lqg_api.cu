@@ -228,6 +228,22 @@ uint32_t batch_visited_bits(const lqg_index* ix, const lqg::ReplayArgs& ra, int6
     return vb;
 }
 
+// Search-heap slots of a batch-kernel launch, `warps` per block: half as many
+// again as the default where they cost no resident block (10,000 queries of
+// integers, 1M x 128 at ef 64 / 500k x 128 at ef 256, ms: 2.07 / 9.35 at 256
+// slots, 2.04 / 9.14 at 384, 2.05 / 9.63 at 512, 2.52 / 10.76 at 1,024: more
+// slots leave less L1, then fewer blocks).
+uint32_t batch_heap_slots(const lqg_index* ix, const lqg::ReplayArgs& ra, uint32_t vbits, int warps) {
+    if (ix->tune.heap_scap != 256) return ra.scap;
+    auto blocks = [&](uint32_t scap) {
+        return 228 * 1024 /
+               (lqg::batch_smem_bytes(ix->dim, ix->deg, vbits, scap, ra.acap, warps) + 1024);
+    };
+    // (registers allow 20 warps per SM)
+    const size_t most = std::min<size_t>(blocks(256), 20 / (size_t)warps);
+    return blocks(384) >= std::max<size_t>(most, 1) ? 384 : ra.scap;
+}
+
 // The same for the latency form with nb blocks per SM, where shared memory is
 // plentiful: first room for the search heap of a query that meets a tie (past
 // its slots in shared memory a push waits for global memory: one tie cost a
@@ -354,7 +370,10 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
             }
             if (cta) latency_shape(ix, nb, h.vbits, ra);
         }
-        if (batch && !cta) h.vbits = batch_visited_bits(ix, ra, b.m, sw);
+        if (batch && !cta) {
+            h.vbits = batch_visited_bits(ix, ra, b.m, sw);
+            ra.scap = batch_heap_slots(ix, ra, h.vbits, sw);
+        }
         if (cta) sw = 1;
         // the batch kernels' distance passes use 4 lanes per candidate; the
         // tuning field keeps its accepted values

@@ -51,9 +51,10 @@ __global__ void entry_distance_kernel(const float* __restrict__ q, int64_t m, ui
 // 6402, 2,368 10081 and 7801, 3,552 10284 and 11287; at 128 and 32, 1,184 blocks:
 // 2,368 3258 and 2566, 4,736 3405 and 2670, 8,192 3659 and 3638. All at ef 512:
 // 888 queries 8473 and 9716; 1,776 at 128 dimensions 3206 and 3288.)
-// The latency form's work list is the queries by descending ef (bins of equal ef,
-// clamped to efmax <= 512, in any order: 9 us for 2,048 queries in one block, where
-// the sort above takes 45).
+// The latency form's work list is the queries by descending ef, counted into bins in
+// one block, in any order within a bin. (A batch that stays with the one-warp form
+// pays 10 to 16 us for this kernel and the other form's empty launch; with the sort
+// above in its place it was 50 to 70.)
 __global__ void __launch_bounds__(1024) choose_form_kernel(const uint32_t* __restrict__ efq,
                                                            uint32_t m, uint32_t efmax,
                                                            uint32_t blocks, int32_t* list,

@@ -53,31 +53,13 @@
 #include <math_constants.h>
 
 #include "heap_ops.cuh"
+#include "launch_shape.h"
 #include "lqg_internal.h"
 #include "lqg_kernels.cuh"
 #include "sq8_batch.cuh"
 #include "sq8_filter.cuh"
 
 namespace lqg {
-
-// Shared memory of one search warp: byte offsets of its parts.
-struct BatchLayout {
-    uint32_t planes, state, vis, cand, heap, pool, popped, total;
-};
-constexpr uint32_t kPoppedBits = 10, kPoppedSlots = 1u << kPoppedBits;
-__host__ __device__ inline BatchLayout batch_layout(uint32_t dim, uint32_t deg, uint32_t vbits,
-                                                    uint32_t scap, uint32_t acap, bool pair = false) {
-    BatchLayout L;
-    L.planes = 4u * ((dim + 15u) & ~15u);            // after the query
-    L.state = L.planes + 2u * filter_plane(dim);     // WarpState
-    L.vis = L.state + 48u;                           // visited cache
-    L.cand = L.vis + (4u << vbits);                  // candidate ids, distances (pair: two)
-    L.heap = L.cand + (pair ? 16u : 8u) * deg;       // search heap
-    L.pool = L.heap + 8u * scap;                     // sorted pool: distances, ids
-    L.popped = L.pool + 8u * acap;                   // pair: popped ids
-    L.total = L.popped + (pair ? 4u * kPoppedSlots : 0u);
-    return L;
-}
 
 // Per-query values that are read once or twice per pop: kept in shared memory,
 // so that the search loop's registers hold only what every step needs.
@@ -185,6 +167,9 @@ struct PairExpand {   // from an expanding warp
     uint32_t mb, mid; // its nearest candidate: distance bits, id
     uint32_t single;  // no other candidate at that distance
 };
+static_assert(sizeof(uint32_t) + 2 * sizeof(PairMerge) + 2 * 3 * sizeof(PairExpand) +
+                      sizeof(uint32_t) + 8 <= kLatencyStatic,
+              "the messages of three expanding warps, the query and the list length");
 constexpr uint32_t kPairFull = 1u;  // rp is full
 constexpr uint32_t kPairTie = 2u;   // another unpopped entry at distance nd
 constexpr uint32_t kPairHeap = 4u;  // the search heap decides every pop

@@ -20,15 +20,4 @@ bool batch_replays_in_place_host(uint32_t deg, uint32_t vbits, uint32_t scap, ui
     return batch_replays_in_place(deg, vbits, scap, acap, rcap);
 }
 
-size_t batch_latency_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t scap,
-                           uint32_t acap) {
-    return 8 * ((dim + 15u) & ~15u) + (size_t)batch_layout(dim, deg, vbits, scap, acap, true).total;
-}
-
-size_t batch_smem_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t scap, uint32_t acap,
-                        int warps) {
-    const size_t dpad = (dim + 15u) & ~15u;
-    return 8 * dpad + (size_t)warps * batch_layout(dim, deg, vbits, scap, acap).total;
-}
-
 }  // namespace lqg

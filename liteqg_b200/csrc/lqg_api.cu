@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "../../include/lqg.h"
+#include "launch_shape.h"
 #include "lqg_build.h"
 #include "lqg_host.h"
 #include "lqg_internal.h"
@@ -197,75 +198,8 @@ lqg_status reset_ctl(Workspace& w, cudaStream_t st) {
     return LQG_OK;
 }
 
-// The tuned search-heap slots, an even number: warps' areas follow each other in
-// shared memory, and their queries are read 16 bytes at a time.
-uint32_t heap_slots(const lqg_tuning& t) { return (t.heap_scap + 1u) & ~1u; }
-
-// The tuned visited-cache bits, or what names the index's ids uniquely
-// (VisitedCache) if that is more.
-uint32_t least_visited_bits(const lqg_index* ix) {
-    uint32_t vb = ix->tune.visited_bits;
-    while (vb < 15 && ix->n > (1ull << (vb + 16))) ++vb;
-    return vb;
-}
-
-// Visited-cache bits of a batch-kernel launch of m queries, `warps` per block.
-// A larger cache forgets fewer nodes (at ef 200 and degree 96: 10.5 k
-// evaluations per query at 10 bits, 6.5 k at 13, 5.6 k without forgetting), but
-// costs resident queries: a batch that fills the GPU runs at the tuned 10 bits
-// (1M x 128, 10,000 queries at ef 64: 2.75 ms at 10, 2.95 at 11, 4.45 at 12).
-// So a batch whose queries all fit at once takes the largest cache they fit
-// with, when the tuning field is at its default; other values are taken as they
-// are.
-uint32_t batch_visited_bits(const lqg_index* ix, const lqg::ReplayArgs& ra, int64_t m, int warps) {
-    const uint32_t vb = least_visited_bits(ix);
-    if (vb != 10) return vb;
-    for (uint32_t x = 13; x > vb; --x) {
-        const size_t smem = lqg::batch_smem_bytes(ix->dim, ix->deg, x, ra.scap, ra.acap, warps);
-        const int64_t per_sm = std::min<int64_t>(228 * 1024 / (smem + 1024), 20 / warps);
-        if (smem <= 227 * 1024 && per_sm * warps * ix->num_sms >= m) return x;
-    }
-    return vb;
-}
-
-// Search-heap slots of a batch-kernel launch, `warps` per block: half as many
-// again as the default where they cost no resident block (10,000 queries of
-// integers, 1M x 128 at ef 64 / 500k x 128 at ef 256, ms: 2.07 / 9.35 at 256
-// slots, 2.04 / 9.14 at 384, 2.05 / 9.63 at 512, 2.52 / 10.76 at 1,024: more
-// slots leave less L1, then fewer blocks).
-uint32_t batch_heap_slots(const lqg_index* ix, const lqg::ReplayArgs& ra, uint32_t vbits, int warps) {
-    if (ix->tune.heap_scap != 256) return ra.scap;
-    auto blocks = [&](uint32_t scap) {
-        return 228 * 1024 /
-               (lqg::batch_smem_bytes(ix->dim, ix->deg, vbits, scap, ra.acap, warps) + 1024);
-    };
-    // (registers allow 20 warps per SM)
-    const size_t most = std::min<size_t>(blocks(256), 20 / (size_t)warps);
-    return blocks(384) >= std::max<size_t>(most, 1) ? 384 : ra.scap;
-}
-
-// The same for the latency form with nb blocks per SM, where shared memory is
-// plentiful: first room for the search heap of a query that meets a tie (past
-// its slots in shared memory a push waits for global memory: one tie cost a
-// query of 560 us another 350 at 256 slots), then the largest visited cache, up
-// to 2^14 (clearing it costs about 600 cycles per query).
-void latency_shape(const lqg_index* ix, int nb, uint32_t& vbits, lqg::ReplayArgs& ra) {
-    const size_t budget = std::min<size_t>(227 * 1024, 228 * 1024 / nb - 1024);
-    auto fits = [&](uint32_t vb, uint32_t scap) {
-        return lqg::batch_latency_bytes(ix->dim, ix->deg, vb, scap, ra.acap) <= budget;
-    };
-    if (ix->tune.heap_scap == 256)
-        for (uint32_t c = 2048; c > 256; c /= 2)
-            if (fits(vbits, c)) {
-                ra.scap = c;
-                break;
-            }
-    if (ix->tune.visited_bits == 10)
-        for (uint32_t x = 14; x > vbits; --x)
-            if (fits(x, ra.scap)) {
-                vbits = x;
-                break;
-            }
+lqg::ShapeIndex shape_index(const lqg_index* ix) {
+    return {ix->dim, ix->deg, ix->n, ix->num_sms, ix->tune};
 }
 
 // Fast kernel over all queries, then the exact kernel over the flagged ones.
@@ -299,7 +233,8 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         lqg::ReplayArgs ra{};
         ra.rcap = (b.ef0 + 2u) & ~1u;
         ra.efcap = std::min(32u * (uint32_t)RE - 32u, ra.rcap - 1u);
-        ra.scap = heap_slots(t);
+        const lqg::ShapeIndex shape = shape_index(ix);
+        ra.scap = lqg::heap_slots(t);
         ra.spill = w.d_spill;
         ra.nspill = w.d_ctl + kCtlSpilled;
         ra.rlog_cap = std::max(1024u, 16u * b.ef0);
@@ -337,7 +272,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         ra.swarps = (uint32_t)sw;
         SearchArgs h = base_args(ix, w, b);
         h.qhead = w.d_ctl + kCtlHeapHead;
-        h.vbits = batch ? least_visited_bits(ix) : t.visited_bits;
+        h.vbits = batch ? lqg::least_visited_bits(shape) : t.visited_bits;
         // small batches: the latency form, when every query of the batch can be
         // resident at once
         bool cta = false;
@@ -348,31 +283,33 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         SearchArgs hl{};
         lqg::ReplayArgs rl{};
         if (batch && b.small_ok && t.small_batch != LQG_SMALL_BATCH_OFF &&
-            lqg::batch_latency_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap) <= 227 * 1024) {
+            lqg::batch_latency_bytes(ix->dim, ix->deg, h.vbits, ra.scap, ra.acap) <= lqg::kBlockBytes) {
             int nb = 1;  // blocks per SM
             if (plain) {
                 cta = true;  // one query: no occupancy question
             } else {
                 int oc = 0;
-                e = lqg::launch_batch_cta(h, ra, degw, 0, b.st, &oc);
-                if (e != cudaSuccess) return cuda_fail(e, "small-batch kernel occupancy");
+                if (lqg::launch_batch_cta(h, ra, degw, 0, b.st, &oc) != cudaSuccess) {
+                    cudaGetLastError();  // the one-warp form takes the batch
+                    oc = 0;
+                }
                 const int64_t lim = t.small_batch == LQG_SMALL_BATCH_AUTO
                                         ? (int64_t)oc * ix->num_sms
                                         : t.small_batch;
                 cta = oc > 0 && b.m <= lim;
                 nb = (int)std::min<int64_t>(oc, (b.m + ix->num_sms - 1) / ix->num_sms);
-                if (!cta && b.efq && t.small_batch == LQG_SMALL_BATCH_AUTO && b.m <= 16 * lim) {
+                if (!cta && oc > 0 && b.efq && t.small_batch == LQG_SMALL_BATCH_AUTO && b.m <= 16 * lim) {
                     lblocks = lim;
                     hl = h;
                     rl = ra;
-                    latency_shape(ix, oc, hl.vbits, rl);
+                    lqg::latency_shape(shape, oc, rl.acap, hl.vbits, rl.scap);
                 }
             }
-            if (cta) latency_shape(ix, nb, h.vbits, ra);
+            if (cta) lqg::latency_shape(shape, nb, ra.acap, h.vbits, ra.scap);
         }
         if (batch && !cta) {
-            h.vbits = batch_visited_bits(ix, ra, b.m, sw);
-            ra.scap = batch_heap_slots(ix, ra, h.vbits, sw);
+            h.vbits = lqg::batch_visited_bits(shape, ra.scap, ra.acap, b.m, sw);
+            ra.scap = lqg::batch_heap_slots(shape, h.vbits, ra.acap, sw);
         }
         if (cta) sw = 1;
         // the batch kernels' distance passes use 4 lanes per candidate; the
@@ -533,7 +470,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         h.vbits = t.visited_bits;
         lqg::HeapArgs hp{};
         hp.rcap = (b.ef0 + 2u) & ~1u;
-        hp.scap = heap_slots(t);
+        hp.scap = lqg::heap_slots(t);
         hp.spill = w.d_spill;
         hp.nspill = w.d_ctl + kCtlSpilled;
         int hw = plain ? 1 : (int)t.heap_warps;

@@ -86,10 +86,6 @@ cudaError_t launch_split(const SearchArgs& a, const ReplayArgs& ra, int E, int G
                          int warps, int blocks, cudaStream_t st, int* occ);
 // Batched-acceptance kernel (batch_kernel.cuh): exact search heap per warp,
 // sorted pool in shared memory, each expansion's candidates decided at once.
-size_t batch_smem_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t scap, uint32_t acap,
-                        int warps);
-// ... of a block of the latency form
-size_t batch_latency_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t scap, uint32_t acap);
 bool batch_replays_in_place_host(uint32_t deg, uint32_t vbits, uint32_t scap, uint32_t acap,
                                  uint32_t rcap);
 cudaError_t launch_batch(const SearchArgs& a, const ReplayArgs& ra, int degw, int warps, int blocks,

@@ -35,6 +35,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "launch_shape.h"
 #include "lqg_kernels.cuh"
 
 namespace lqg {
@@ -43,9 +44,6 @@ constexpr float kFilterRel = 1.00004f;
 
 // Rows of at least this many code bytes ("wide") prefetch along the row.
 constexpr uint32_t kWideDim = 256;
-
-// Bytes of one plane of a query: whole rounds of two 64-byte slices, zero past dim.
-__host__ __device__ inline uint32_t filter_plane(uint32_t dim) { return (dim + 127u) & ~127u; }
 
 struct Sq8Filter {
     float K;   // sum t^2 + 128 sum r

@@ -1,0 +1,105 @@
+"""The batch kernel's launch shapes (csrc/launch_shape.h): what the host chooses
+fits an SM as the hardware counts it."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SM, BLOCK, OWN, UNIT = 228 * 1024, 227 * 1024, 1024, 128  # shared memory of an SM and of a block
+
+PROGRAM = r"""
+#include <cstdio>
+#include <cstring>
+#include "launch_shape.h"
+using namespace lqg;
+int main() {
+    char op[16];
+    unsigned dim, deg, vb, scap, tv, ts, acap;
+    unsigned long long n;
+    long long m;
+    int w;
+    // op, index, tuning fields, shape so far, queries, warps (blocks per SM for "latency")
+    while (std::scanf("%15s %u %u %llu %u %u %u %u %u %lld %d", op, &dim, &deg, &n, &tv, &ts, &vb,
+                      &scap, &acap, &m, &w) == 11) {
+        ShapeIndex x{};
+        x.dim = dim, x.deg = deg, x.n = n, x.sms = 148;
+        x.t.visited_bits = tv, x.t.heap_scap = ts;
+        size_t bytes = 0;
+        if (!std::strcmp(op, "latency")) {
+            latency_shape(x, w, acap, vb, scap);
+            bytes = 8 * ((dim + 15u) & ~15u) + batch_layout(dim, deg, vb, scap, acap, true).total;
+        }
+        std::printf("%u %u %zu\n", vb, scap, bytes);
+    }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def shapes(tmp_path_factory):
+    """Runs the rules on rows (op, dim, deg, n, tuned visited bits, tuned slots,
+    bits, slots, pool slots, queries, warps): rows of (bits, slots, bytes)."""
+    d = tmp_path_factory.mktemp("shape")
+    (d / "main.cpp").write_text(PROGRAM)
+    exe = str(d / "shape")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "liteqg_b200", "csrc"),
+                    str(d / "main.cpp"), "-o", exe], check=True)
+
+    def run(rows):
+        text = "\n".join(" ".join(str(v) for v in r) for r in rows) + "\n"
+        out = subprocess.run([exe], input=text, capture_output=True, text=True, check=True).stdout
+        return np.array([[int(v) for v in line.split()] for line in out.splitlines()])
+
+    return run
+
+
+def _own(dynamic, static):
+    """What a resident block takes of an SM."""
+    return -(-(dynamic + static + OWN) // UNIT) * UNIT
+
+
+@pytest.mark.parametrize("deg", [32, 64, 96, 128])
+def test_latency_blocks_fit_with_their_messages(shapes, deg):
+    static = 176  # the kernel's own __shared__ variables, three expanding warps
+    rows, most = [], []
+    for dim in (33, 96, 100, 128, 300, 768, 960, 1536, 2048):
+        for acap in (96, 128, 192, 320, 576):
+            for scap in (256, 4096, 13000, 16376, 16384):
+                # resident blocks at the smallest shape, as the occupancy query counts them
+                base = 8 * (-(-dim // 16) * 16)
+                base += 4 * (-(-dim // 16) * 16) + 2 * (-(-dim // 128) * 128) + 48 + 4096
+                base += 16 * deg + 8 * scap + 8 * acap + 4096
+                if base + static > BLOCK:
+                    continue
+                for nb in range(1, min(8, SM // _own(base, static)) + 1):
+                    rows.append(("latency", dim, deg, 100000, 10, scap, 10, scap, acap, 1, nb))
+                    most.append(nb)
+    got = shapes(rows)
+    for row, nb, (_, _, dynamic) in zip(rows, most, got):
+        assert dynamic + static <= BLOCK, row
+        assert nb * _own(dynamic, static) <= SM, row
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 5, 200])
+def test_large_rows_and_heaps(m):
+    """The largest rows beside a search heap that nearly fills a block."""
+    import liteqg_b200
+    from oracle.oracle import IndexArrays, Oracle, sq8_quantize
+
+    rng = np.random.default_rng(m)
+    n, dim, deg, k, ef = 600, 2048, 32, 10, 200
+    x = rng.integers(0, 24, (n, dim)).astype(np.float32)
+    q = rng.integers(0, 24, (m, dim)).astype(np.float32)
+    nb = np.stack([rng.choice(n, deg, replace=False) for _ in range(n)]).astype(np.uint32)
+    codes, params = sq8_quantize(x, 2)
+    ix = liteqg_b200.Index("QG", "L2", n, dim, deg)
+    ix.set_arrays(7, x, nb, codes, params)
+    ix.set_tuning(heap_scap=16376)
+    want = Oracle(IndexArrays(n, dim, deg, 7, x, nb, codes, params)).search(q, k, ef).compat
+    if m == 1:
+        ix.set_ef(ef)
+        assert np.array_equal(ix.search(q[0], k), want[0])
+    assert np.array_equal(ix.search(q, k, ef=ef), want)

@@ -216,7 +216,7 @@ constexpr uint32_t kPairRedo = 16u; // the step's expansion does not count; expa
 //   100k x 960 deg 64 ef 32-512, 2,048        20,550 -> 10,970
 //   100k x 100 deg 96 ef 200, 1,777 queries    3,016 -> 2,334
 template <int DEGW, bool WIDE, int NE>
-__global__ void __maxnreg__(WIDE || NE ? 128 : 96)
+__global__ void __maxnreg__(WIDE || NE ? kWideRegs : kNarrowRegs)
     batch_search_kernel(const __grid_constant__ SearchArgs a, const __grid_constant__ ReplayArgs ra) {
     using namespace heapops;
     extern __shared__ __align__(16) unsigned char smem[];

@@ -22,6 +22,12 @@ namespace lqg {
 constexpr size_t kBlockBytes = 227 * 1024;
 constexpr size_t kSmBytes = 228 * 1024;
 constexpr size_t kBlockOwn = 1024, kBlockUnit = 128;
+constexpr uint32_t kSmRegs = 65536;
+
+// Rows of at least this many code bytes ("wide") prefetch along the row; the
+// batch kernel's instances for them take more registers.
+constexpr uint32_t kWideDim = 256;
+constexpr uint32_t kNarrowRegs = 96, kWideRegs = 128;  // per thread (batch_kernel.cuh)
 
 // Bytes of one plane of a query's distance bound (sq8_filter.cuh): whole rounds
 // of two 64-byte slices, zero past dim.
@@ -69,6 +75,16 @@ struct ShapeIndex {
     lqg_tuning t;
 };
 
+// Resident blocks of `warps` query warps per SM, by shared memory and registers.
+inline int64_t batch_blocks(const ShapeIndex& x, uint32_t vbits, uint32_t scap, uint32_t acap,
+                            int warps) {
+    const size_t smem = batch_smem_bytes(x.dim, x.deg, vbits, scap, acap, warps);
+    if (smem > kBlockBytes) return 0;
+    const uint32_t regs = x.dim >= kWideDim ? kWideRegs : kNarrowRegs;
+    return std::min<int64_t>(kSmBytes / ((smem + kBlockOwn + kBlockUnit - 1) / kBlockUnit * kBlockUnit),
+                             kSmRegs / (regs * 32 * (uint32_t)warps));
+}
+
 // The tuned search-heap slots, an even number: warps' areas follow each other in
 // shared memory, and their queries are read 16 bytes at a time.
 inline uint32_t heap_slots(const lqg_tuning& t) { return (t.heap_scap + 1u) & ~1u; }
@@ -93,11 +109,8 @@ inline uint32_t batch_visited_bits(const ShapeIndex& x, uint32_t scap, uint32_t 
                                    int warps) {
     const uint32_t vb = least_visited_bits(x);
     if (vb != 10) return vb;
-    for (uint32_t b = 13; b > vb; --b) {
-        const size_t smem = batch_smem_bytes(x.dim, x.deg, b, scap, acap, warps);
-        const int64_t per_sm = std::min<int64_t>(kSmBytes / (smem + kBlockOwn), 20 / warps);
-        if (smem <= kBlockBytes && per_sm * warps * x.sms >= m) return b;
-    }
+    for (uint32_t b = 13; b > vb; --b)
+        if (batch_blocks(x, b, scap, acap, warps) * warps * x.sms >= m) return b;
     return vb;
 }
 
@@ -108,12 +121,8 @@ inline uint32_t batch_visited_bits(const ShapeIndex& x, uint32_t scap, uint32_t 
 // slots leave less L1, then fewer blocks).
 inline uint32_t batch_heap_slots(const ShapeIndex& x, uint32_t vbits, uint32_t acap, int warps) {
     if (x.t.heap_scap != 256) return heap_slots(x.t);
-    auto blocks = [&](uint32_t scap) {
-        return kSmBytes / (batch_smem_bytes(x.dim, x.deg, vbits, scap, acap, warps) + kBlockOwn);
-    };
-    // (registers allow 20 warps per SM)
-    const size_t most = std::min<size_t>(blocks(256), 20 / (size_t)warps);
-    return blocks(384) >= std::max<size_t>(most, 1) ? 384 : 256;
+    const int64_t least = std::max<int64_t>(batch_blocks(x, vbits, 256, acap, warps), 1);
+    return batch_blocks(x, vbits, 384, acap, warps) >= least ? 384 : 256;
 }
 
 // The same for the latency form with nb blocks per SM, where shared memory is

@@ -42,9 +42,6 @@ namespace lqg {
 
 constexpr float kFilterRel = 1.00004f;
 
-// Rows of at least this many code bytes ("wide") prefetch along the row.
-constexpr uint32_t kWideDim = 256;
-
 struct Sq8Filter {
     float K;   // sum t^2 + 128 sum r
     float st;  // step of G

@@ -30,6 +30,10 @@ int main() {
         if (!std::strcmp(op, "latency")) {
             latency_shape(x, w, acap, vb, scap);
             bytes = 8 * ((dim + 15u) & ~15u) + batch_layout(dim, deg, vb, scap, acap, true).total;
+        } else {
+            if (!std::strcmp(op, "bits")) vb = batch_visited_bits(x, scap, acap, m, w);
+            if (!std::strcmp(op, "slots")) scap = batch_heap_slots(x, vb, acap, w);
+            bytes = batch_smem_bytes(dim, deg, vb, scap, acap, w);
         }
         std::printf("%u %u %zu\n", vb, scap, bytes);
     }
@@ -80,6 +84,32 @@ def test_latency_blocks_fit_with_their_messages(shapes, deg):
     for row, nb, (_, _, dynamic) in zip(rows, most, got):
         assert dynamic + static <= BLOCK, row
         assert nb * _own(dynamic, static) <= SM, row
+
+
+def _blocks(dim, warps, dynamic):
+    """Resident blocks of the one-warp form: registers per thread as compiled."""
+    regs = 128 if dim >= 256 else 96
+    return min(SM // _own(dynamic, 0), 65536 // (regs * 32 * warps))
+
+
+@pytest.mark.parametrize("warps", [1, 2, 3, 4, 5])
+def test_more_slots_and_bits_only_where_they_are_free(shapes, warps):
+    cases = [(dim, deg, acap) for dim in (33, 96, 128, 255, 256, 300, 384, 400, 512, 768, 960, 2048)
+             for deg in (32, 64, 128) for acap in (96, 128, 192, 320, 576)]
+    plain, more, chosen, bits = (shapes([(op, dim, deg, 100000, 10, 256, 10, s, acap, m, warps)
+                                         for dim, deg, acap in cases])
+                                 for op, s, m in (("bytes", 256, 1), ("bytes", 384, 1),
+                                                  ("slots", 256, 1), ("bits", 256, 1500)))
+    for (dim, deg, acap), p, q, c, b in zip(cases, plain, more, chosen, bits):
+        before = _blocks(dim, warps, p[2])
+        if before < 1:
+            continue
+        free = q[2] <= BLOCK and _blocks(dim, warps, q[2]) >= before
+        assert (c[1] == 384) == free, (dim, deg, acap)
+        resident = [_blocks(dim, warps, p[2] + warps * ((4 << x) - 4096)) * warps * 148
+                    for x in (11, 12, 13)]
+        fits = [x for x, r in zip((11, 12, 13), resident) if r >= 1500]
+        assert b[0] == (max(fits) if fits else 10), (dim, deg, acap)
 
 
 @pytest.mark.gpu

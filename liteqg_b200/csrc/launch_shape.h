@@ -97,6 +97,17 @@ inline uint32_t least_visited_bits(const ShapeIndex& x) {
     return vb;
 }
 
+// Warps of a batch-kernel block, at most `warps`, so that the block launches at the
+// least visited bits. (With ids past 2^29 the cache alone may leave too little for
+// the tuned slots of a single warp; the heap then spills to global memory earlier.)
+inline int batch_warps(const ShapeIndex& x, uint32_t acap, int warps, uint32_t& scap) {
+    const uint32_t vb = least_visited_bits(x);
+    auto fits = [&] { return batch_smem_bytes(x.dim, x.deg, vb, scap, acap, warps) <= kBlockBytes; };
+    while (warps > 1 && !fits()) --warps;
+    while (scap > 256 && !fits()) scap = std::max(256u, scap / 2 & ~1u);
+    return warps;
+}
+
 // Visited-cache bits of a batch-kernel launch of m queries, `warps` per block.
 // A larger cache forgets fewer nodes (at ef 200 and degree 96: 10.5 k
 // evaluations per query at 10 bits, 6.5 k at 13, 5.6 k without forgetting), but
@@ -119,8 +130,9 @@ inline uint32_t batch_visited_bits(const ShapeIndex& x, uint32_t scap, uint32_t 
 // integers, 1M x 128 at ef 64 / 500k x 128 at ef 256, ms: 2.07 / 9.35 at 256
 // slots, 2.04 / 9.14 at 384, 2.05 / 9.63 at 512, 2.52 / 10.76 at 1,024: more
 // slots leave less L1, then fewer blocks).
-inline uint32_t batch_heap_slots(const ShapeIndex& x, uint32_t vbits, uint32_t acap, int warps) {
-    if (x.t.heap_scap != 256) return heap_slots(x.t);
+inline uint32_t batch_heap_slots(const ShapeIndex& x, uint32_t vbits, uint32_t scap, uint32_t acap,
+                                 int warps) {
+    if (x.t.heap_scap != 256) return scap;
     const int64_t least = std::max<int64_t>(batch_blocks(x, vbits, 256, acap, warps), 1);
     return batch_blocks(x, vbits, 384, acap, warps) >= least ? 384 : 256;
 }

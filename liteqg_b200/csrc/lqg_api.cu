@@ -259,9 +259,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         // split kernel blocks hold at most 5 warps (its 96-register budget)
         int sw = plain ? 1 : (int)(split ? std::min(t.heap_warps, 5u) : t.replay_warps);
         if (batch) {
-            while (sw > 1 &&
-                   lqg::batch_smem_bytes(ix->dim, ix->deg, t.visited_bits, ra.scap, ra.acap, sw) > 227 * 1024)
-                --sw;
+            sw = lqg::batch_warps(shape, ra.acap, sw, ra.scap);
         } else if (split) {
             while (sw > 1 && lqg::split_smem_bytes(ix->dim, t.visited_bits, ra.scap, sw) > 227 * 1024)
                 --sw;
@@ -309,7 +307,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         }
         if (batch && !cta) {
             h.vbits = lqg::batch_visited_bits(shape, ra.scap, ra.acap, b.m, sw);
-            ra.scap = lqg::batch_heap_slots(shape, h.vbits, ra.acap, sw);
+            ra.scap = lqg::batch_heap_slots(shape, h.vbits, ra.scap, ra.acap, sw);
         }
         if (cta) sw = 1;
         // the batch kernels' distance passes use 4 lanes per candidate; the

@@ -31,8 +31,14 @@ int main() {
             latency_shape(x, w, acap, vb, scap);
             bytes = 8 * ((dim + 15u) & ~15u) + batch_layout(dim, deg, vb, scap, acap, true).total;
         } else {
+            if (!std::strcmp(op, "launch")) {  // as run_batch goes about it
+                std::printf("%zu ", batch_smem_bytes(dim, deg, tv, ts, 32 * 17, 1));  // set_tuning's
+                w = batch_warps(x, acap, w, scap);
+                vb = batch_visited_bits(x, scap, acap, m, w);
+                scap = batch_heap_slots(x, vb, scap, acap, w);
+            }
             if (!std::strcmp(op, "bits")) vb = batch_visited_bits(x, scap, acap, m, w);
-            if (!std::strcmp(op, "slots")) scap = batch_heap_slots(x, vb, acap, w);
+            if (!std::strcmp(op, "slots")) scap = batch_heap_slots(x, vb, scap, acap, w);
             bytes = batch_smem_bytes(dim, deg, vb, scap, acap, w);
         }
         std::printf("%u %u %zu\n", vb, scap, bytes);
@@ -110,6 +116,19 @@ def test_more_slots_and_bits_only_where_they_are_free(shapes, warps):
                     for x in (11, 12, 13)]
         fits = [x for x, r in zip((11, 12, 13), resident) if r >= 1500]
         assert b[0] == (max(fits) if fits else 10), (dim, deg, acap)
+
+
+@pytest.mark.parametrize("n", [100000, 2**24, 2**24 + 1, 2**26 + 1, 2**28, 2**29 + 1, 2**31 - 1])
+def test_many_ids_need_more_bits_and_still_fit(shapes, n):
+    """Every tuning that set_tuning takes launches, whatever the ids need."""
+    rows = [("launch", dim, deg, n, tv, ts, 0, ts, acap, 100000, warps)
+            for dim in (33, 128, 960, 2048) for deg in (32, 128) for acap in (96, 320, 576)
+            for tv in (8, 10, 13) for ts in (256, 1024, 2500, 4096, 9000, 16384) for warps in (1, 3, 5)]
+    for row, (accepted, bits, slots, dynamic) in zip(rows, shapes(rows)):
+        if accepted > BLOCK:
+            continue
+        assert dynamic <= BLOCK and slots >= 256, row
+        assert n <= 1 << (bits + 16), row  # slot and tag name one id
 
 
 @pytest.mark.gpu

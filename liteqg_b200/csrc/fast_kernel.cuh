@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include "launch_shape.h"
 #include "lqg_internal.h"
 #include "lqg_kernels.cuh"
 #include "sq8_batch.cuh"
@@ -50,15 +51,6 @@ __device__ __forceinline__ float pool_at(const float (&pd)[E], uint32_t lane_of,
     for (int t = 1; t < E; ++t)
         if (slot_of == (uint32_t)t) v = pd[t];
     return __shfl_sync(kFull, v, lane_of);
-}
-
-// Shared memory of one warp: the query, its byte planes, the cache of evaluated
-// nodes, the place cache (lists of several words), candidate ids, distances and
-// places.
-__host__ __device__ inline uint32_t fast_warp_bytes(uint32_t dim, uint32_t deg, uint32_t vbits,
-                                                    uint32_t sbits) {
-    return 4u * ((dim + 15u) & ~15u) + 2u * filter_plane(dim) + (4u << sbits) +
-           (deg > 32 ? 4u << vbits : 0u) + 12u * deg;
 }
 
 template <int E, int DEGW>

@@ -14,10 +14,6 @@ extern template cudaError_t fast_dispatch<8>(const SearchArgs&, int, int, int, s
 extern template cudaError_t fast_dispatch<16>(const SearchArgs&, int, int, int, size_t,
                                               cudaStream_t, int*);
 
-size_t fast_smem_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t sbits, int warps) {
-    return 8 * ((dim + 15u) & ~15u) + (size_t)warps * fast_warp_bytes(dim, deg, vbits, sbits);
-}
-
 static cudaError_t dispatch(const SearchArgs& a, int E, int degw, int warps, int blocks,
                             size_t smem, cudaStream_t st, int* occ) {
     switch (E) {

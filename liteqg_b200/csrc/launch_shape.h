@@ -163,4 +163,30 @@ inline void latency_shape(const ShapeIndex& x, int nb, uint32_t acap, uint32_t& 
             }
 }
 
+// Shared memory of a warp of the fast kernel: the query, its byte planes, the cache
+// of evaluated nodes, the place cache (lists of several words), candidate ids,
+// distances and places; and of a block.
+LQG_HD inline uint32_t fast_warp_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t sbits) {
+    return 4u * ((dim + 15u) & ~15u) + 2u * filter_plane(dim) + (4u << sbits) +
+           (deg > 32 ? 4u << vbits : 0u) + 12u * deg;
+}
+inline size_t fast_smem_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t sbits, int warps) {
+    return 8 * (size_t)((dim + 15u) & ~15u) +
+           (size_t)warps * fast_warp_bytes(dim, deg, vbits, sbits);
+}
+
+// The fewest bits of its cache of evaluated nodes: 9, or what names the index's ids
+// uniquely; and the warps of a block, at most `warps`, that launches with them.
+inline uint32_t least_seen_bits(const ShapeIndex& x) {
+    uint32_t sb = 9;
+    while (sb < 15 && x.n > (1ull << (sb + 16))) ++sb;
+    return sb;
+}
+inline int fast_warps(const ShapeIndex& x, int warps) {
+    while (warps > 1 && fast_smem_bytes(x.dim, x.deg, x.t.visited_bits, least_seen_bits(x), warps) >
+                            kBlockBytes)
+        --warps;
+    return warps;
+}
+
 }  // namespace lqg

@@ -426,15 +426,12 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         a.path = b.path;
         a.path_stride = b.path_stride;
         a.qlist = order;
-        int warps = plain ? 1 : (int)t.warps_per_block;
-        while (warps > 1 &&
-               lqg::fast_smem_bytes(ix->dim, ix->deg, a.vbits, 9, warps) > 227 * 1024)
-            --warps;
+        const lqg::ShapeIndex shape = shape_index(ix);
+        const int warps = plain ? 1 : lqg::fast_warps(shape, (int)t.warps_per_block);
         // The cache of evaluated nodes: the largest that costs no resident
         // warps (each node that it forgets is bounded again, once per pop that
         // lists it); at least what names the index's ids uniquely.
-        uint32_t smin = 9;
-        while (smin < 15 && ix->n > (1ull << (smin + 16))) ++smin;
+        const uint32_t smin = lqg::least_seen_bits(shape);
         a.sbits = plain ? std::max(smin, 12u) : smin;
         int blocks = 1;
         if (!plain) {

@@ -14,7 +14,6 @@ cudaError_t launch_fast(const SearchArgs& a, int E, int degw, int warps, int blo
                         cudaStream_t st);
 // Resident blocks per SM for that instance (0 if it cannot launch).
 int fast_occupancy(int E, int degw, int warps, uint32_t dim, uint32_t vbits, uint32_t sbits);
-size_t fast_smem_bytes(uint32_t dim, uint32_t deg, uint32_t vbits, uint32_t sbits, int warps);
 
 // One launch of the exact kernel over a work list; blocks*warps must equal
 // the number of scratch slots in s.

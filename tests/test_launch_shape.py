@@ -30,6 +30,10 @@ int main() {
         if (!std::strcmp(op, "latency")) {
             latency_shape(x, w, acap, vb, scap);
             bytes = 8 * ((dim + 15u) & ~15u) + batch_layout(dim, deg, vb, scap, acap, true).total;
+        } else if (!std::strcmp(op, "fast")) {
+            w = fast_warps(x, w);
+            vb = least_seen_bits(x);
+            bytes = fast_smem_bytes(dim, deg, tv, vb, w);
         } else {
             if (!std::strcmp(op, "launch")) {  // as run_batch goes about it
                 std::printf("%zu ", batch_smem_bytes(dim, deg, tv, ts, 32 * 17, 1));  // set_tuning's
@@ -129,6 +133,15 @@ def test_many_ids_need_more_bits_and_still_fit(shapes, n):
             continue
         assert dynamic <= BLOCK and slots >= 256, row
         assert n <= 1 << (bits + 16), row  # slot and tag name one id
+
+
+@pytest.mark.parametrize("n", [100000, 2**25 + 1, 2**26 + 1, 2**31 - 1])
+def test_fast_kernel_fits_with_many_ids(shapes, n):
+    rows = [("fast", dim, deg, n, tv, 256, 0, 0, 0, 1, warps)
+            for dim in (33, 400, 960, 1000, 2048) for deg in (32, 64) for tv in (8, 10, 13)
+            for warps in (1, 8, 16)]
+    for row, (bits, _, dynamic) in zip(rows, shapes(rows)):
+        assert dynamic <= BLOCK and n <= 1 << (bits + 16), row
 
 
 @pytest.mark.gpu

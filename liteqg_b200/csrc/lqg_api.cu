@@ -275,8 +275,8 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         // resident at once
         bool cta = false;
         // resident blocks of the latency form, if a device-side look at the
-        // queries' ef shall choose between the forms (choose_form_kernel; past 16
-        // per block it would hardly choose this one)
+        // queries' ef may choose between the forms (choose_form_kernel; past 16
+        // per block it would hardly choose this one): with per-query ef
         int64_t lblocks = 0;
         SearchArgs hl{};
         lqg::ReplayArgs rl{};
@@ -296,7 +296,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
                                         : t.small_batch;
                 cta = oc > 0 && b.m <= lim;
                 nb = (int)std::min<int64_t>(oc, (b.m + ix->num_sms - 1) / ix->num_sms);
-                if (!cta && oc > 0 && b.efq && t.small_batch == LQG_SMALL_BATCH_AUTO && b.m <= 16 * lim) {
+                if (!cta && oc > 0 && t.small_batch == LQG_SMALL_BATCH_AUTO && b.m <= 16 * lim) {
                     lblocks = lim;
                     hl = h;
                     rl = ra;
@@ -334,8 +334,9 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
         // longest-expected queries first, when a chunk holds more queries
         // than the launch has warps (otherwise they all start at once)
         const bool order = !plain && chunk > (int64_t)rb * sw;
-        // (a later batch with per-query ef may need a work list)
-        if ((order || (batch && b.efq)) && (s = ensure_order(w, chunk)) != LQG_OK) return s;
+        // (with or without per-query ef: a batch of the same size that is captured
+        // later may have one, and allocates nothing)
+        if ((order || lblocks > 0) && (s = ensure_order(w, chunk)) != LQG_OK) return s;
         const size_t slots = std::max((size_t)rb * sw, (size_t)lblocks);
         if (w.sp_global_slots < slots) {
             dfree(w.d_sp_global);
@@ -371,7 +372,7 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
                 (s = order_queries(ix, w, c.queries, c.efq, mc, b.st, &c.qlist)) != LQG_OK)
                 return s;
             const int cb = (int)std::min<int64_t>(rb, (mc + sw - 1) / sw);
-            if (lblocks > 0) {
+            if (lblocks > 0 && b.efq) {
                 const int32_t* warp_list = c.qlist;
                 if ((s = choose_form(w, c.efq, mc, b.ef0, lblocks, b.st, &c.qlist)) != LQG_OK)
                     return s;

@@ -1324,20 +1324,23 @@ LQG_API lqg_status lqg_fs_search_batch(lqg_index* ix, const float* queries, int6
         st = ix->own_stream;
     }
     if ((s = grow(w.d_q, w.cap_q, (size_t)m * ix->dim)) != LQG_OK) return s;
-    if ((s = grow(w.d_ids, w.cap_ids, (size_t)m * kstride)) != LQG_OK) return s;
+    uint32_t* d_ids = nullptr;
+    if ((s = ensure_ctl(w, 0)) != LQG_OK) return s;
+    if ((s = ids_area(w, (size_t)m * kstride, &d_ids)) != LQG_OK) return s;
     if (k && (s = grow(w.d_kq, w.cap_kq, (size_t)m)) != LQG_OK) return s;
     if (ef && (s = grow(w.d_efq, w.cap_efq, (size_t)m)) != LQG_OK) return s;
     if (stats && (s = grow(w.d_stats, w.cap_stats, (size_t)m * 4)) != LQG_OK) return s;
-    if ((s = copy_in(w, w.d_q, queries, (size_t)m * ix->dim * 4, st)) != LQG_OK) return s;
-    if (k && (s = copy_in(w, w.d_kq, k, m * 4, st)) != LQG_OK) return s;
-    if (ef && (s = copy_in(w, w.d_efq, ef, m * 4, st)) != LQG_OK) return s;
-    s = fs_run(ix, w, w.d_q, m, k ? w.d_kq : nullptr, k0, ef ? w.d_efq : nullptr, efb, w.d_ids,
+    LQG_CUDA(cudaMemcpyAsync(w.d_q, queries, (size_t)m * ix->dim * 4, cudaMemcpyHostToDevice, st));
+    if (k) LQG_CUDA(cudaMemcpyAsync(w.d_kq, k, m * 4, cudaMemcpyHostToDevice, st));
+    if (ef) LQG_CUDA(cudaMemcpyAsync(w.d_efq, ef, m * 4, cudaMemcpyHostToDevice, st));
+    s = fs_run(ix, w, w.d_q, m, k ? w.d_kq : nullptr, k0, ef ? w.d_efq : nullptr, efb, d_ids,
                kstride, stats ? w.d_stats : nullptr, st, m == 1);
     if (s != LQG_OK) return s;
-    if ((s = fetch_ctl(w, std::max<size_t>(kstride, 4u) * (size_t)m * 4, st)) != LQG_OK) return s;
-    if ((s = copy_out(w, ids, w.d_ids, (size_t)m * kstride * 4, st)) != LQG_OK) return s;
-    if (stats && (s = copy_out(w, stats, w.d_stats, (size_t)m * 16, st)) != LQG_OK) return s;
-    return fs_status_of(w.stage.ctl());
+    if (stats)
+        LQG_CUDA(cudaMemcpyAsync(stats, w.d_stats, (size_t)m * 16, cudaMemcpyDeviceToHost, st));
+    uint32_t ctl[kCtlWords];
+    if ((s = fetch_ids(w, ids, (size_t)m * kstride, ctl, st)) != LQG_OK) return s;
+    return fs_status_of(ctl);
 }
 
 LQG_API lqg_status lqg_selftest_bounded_wait(int device, uint32_t tries, uint32_t* timed_out) {

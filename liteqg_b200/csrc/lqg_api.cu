@@ -100,7 +100,7 @@ int pool_regs_for(uint32_t ef_max) {
 
 lqg_status ensure_ctl(Workspace& w, int64_t m) {
     if (!w.d_ctl) {
-        if (cudaMalloc(&w.d_ctl, kCtlWords * sizeof(uint32_t)) != cudaSuccess) {
+        if (cudaMalloc(&w.d_ctl, (kCtlWords + kNearIds) * sizeof(uint32_t)) != cudaSuccess) {
             cudaGetLastError();
             return fail(LQG_ERR_NOMEM, "control block allocation failed");
         }
@@ -533,6 +533,36 @@ lqg_status read_status(Workspace& w, cudaStream_t st) {
     return status_of(ctl);
 }
 
+lqg_status ids_area(Workspace& w, size_t n, uint32_t** area) {
+    if (n <= kNearIds) {
+        *area = w.d_ctl + kCtlWords;
+        return LQG_OK;
+    }
+    lqg_status s = grow(w.d_ids, w.cap_ids, n);
+    *area = w.d_ids;
+    return s;
+}
+
+lqg_status fetch_ids(Workspace& w, uint32_t* ids, size_t n, uint32_t (&ctl)[kCtlWords],
+                     cudaStream_t st) {
+    const bool near = n <= kNearIds;
+    if (near && !w.h_near)
+        w.h_near = static_cast<uint32_t*>(std::malloc((kCtlWords + kNearIds) * sizeof(uint32_t)));
+    if (near && w.h_near) {
+        LQG_CUDA(cudaMemcpyAsync(w.h_near, w.d_ctl, (kCtlWords + n) * sizeof(uint32_t),
+                                 cudaMemcpyDeviceToHost, st));
+        LQG_CUDA(cudaStreamSynchronize(st));
+        std::memcpy(ctl, w.h_near, sizeof(ctl));
+        if (n) std::memcpy(ids, w.h_near + kCtlWords, n * sizeof(uint32_t));
+        return LQG_OK;
+    }
+    LQG_CUDA(cudaMemcpyAsync(ids, near ? w.d_ctl + kCtlWords : w.d_ids, n * sizeof(uint32_t),
+                             cudaMemcpyDeviceToHost, st));
+    LQG_CUDA(cudaMemcpyAsync(ctl, w.d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st));
+    LQG_CUDA(cudaStreamSynchronize(st));
+    return LQG_OK;
+}
+
 // Host-buffer batch: copy in, search, copy out, wait (one workspace).
 lqg_status search_host(lqg_index* ix, Workspace& w, const float* queries, int64_t m,
                        const uint32_t* k, uint32_t k0, const uint32_t* ef, uint32_t efb,
@@ -540,7 +570,9 @@ lqg_status search_host(lqg_index* ix, Workspace& w, const float* queries, int64_
                        uint32_t pstride, uint32_t* stats, cudaStream_t st) {
     lqg_status s;
     if ((s = grow(w.d_q, w.cap_q, (size_t)m * ix->dim)) != LQG_OK) return s;
-    if ((s = grow(w.d_ids, w.cap_ids, (size_t)m * kstride)) != LQG_OK) return s;
+    uint32_t* d_ids = nullptr;
+    if ((s = ensure_ctl(w, 0)) != LQG_OK) return s;
+    if ((s = ids_area(w, (size_t)m * kstride, &d_ids)) != LQG_OK) return s;
     if (k && (s = grow(w.d_kq, w.cap_kq, (size_t)m)) != LQG_OK) return s;
     if (ef && (s = grow(w.d_efq, w.cap_efq, (size_t)m)) != LQG_OK) return s;
     if (stats && (s = grow(w.d_stats, w.cap_stats, (size_t)m * 4)) != LQG_OK) return s;
@@ -548,16 +580,16 @@ lqg_status search_host(lqg_index* ix, Workspace& w, const float* queries, int64_
         if ((s = grow(w.d_pool_ids, w.cap_pool_ids, (size_t)m * pstride)) != LQG_OK) return s;
         if ((s = grow(w.d_pool_d, w.cap_pool_d, (size_t)m * pstride)) != LQG_OK) return s;
     }
-    if ((s = copy_in(w, w.d_q, queries, (size_t)m * ix->dim * 4, st)) != LQG_OK) return s;
-    if (k && (s = copy_in(w, w.d_kq, k, m * 4, st)) != LQG_OK) return s;
-    if (ef && (s = copy_in(w, w.d_efq, ef, m * 4, st)) != LQG_OK) return s;
+    LQG_CUDA(cudaMemcpyAsync(w.d_q, queries, (size_t)m * ix->dim * 4, cudaMemcpyHostToDevice, st));
+    if (k) LQG_CUDA(cudaMemcpyAsync(w.d_kq, k, m * 4, cudaMemcpyHostToDevice, st));
+    if (ef) LQG_CUDA(cudaMemcpyAsync(w.d_efq, ef, m * 4, cudaMemcpyHostToDevice, st));
     BatchSpec b{w.d_q,
                 m,
                 k ? w.d_kq : nullptr,
                 k0,
                 ef ? w.d_efq : nullptr,
                 efb,
-                w.d_ids,
+                d_ids,
                 kstride,
                 pool_ids ? w.d_pool_ids : nullptr,
                 pool_ids ? w.d_pool_d : nullptr,
@@ -565,15 +597,17 @@ lqg_status search_host(lqg_index* ix, Workspace& w, const float* queries, int64_
                 stats ? w.d_stats : nullptr,
                 st};
     if ((s = run_batch(ix, w, b, false)) != LQG_OK) return s;
-    const size_t most = std::max<size_t>(std::max(kstride, pool_ids ? pstride : 0u), 4u) * (size_t)m * 4;
-    if ((s = fetch_ctl(w, most, st)) != LQG_OK) return s;
-    if ((s = copy_out(w, ids, w.d_ids, (size_t)m * kstride * 4, st)) != LQG_OK) return s;
     if (pool_ids) {
-        if ((s = copy_out(w, pool_ids, w.d_pool_ids, (size_t)m * pstride * 4, st)) != LQG_OK) return s;
-        if ((s = copy_out(w, pool_d, w.d_pool_d, (size_t)m * pstride * 4, st)) != LQG_OK) return s;
+        LQG_CUDA(cudaMemcpyAsync(pool_ids, w.d_pool_ids, (size_t)m * pstride * 4,
+                                 cudaMemcpyDeviceToHost, st));
+        LQG_CUDA(cudaMemcpyAsync(pool_d, w.d_pool_d, (size_t)m * pstride * 4,
+                                 cudaMemcpyDeviceToHost, st));
     }
-    if (stats && (s = copy_out(w, stats, w.d_stats, (size_t)m * 16, st)) != LQG_OK) return s;
-    return status_of(w.stage.ctl());
+    if (stats)
+        LQG_CUDA(cudaMemcpyAsync(stats, w.d_stats, (size_t)m * 16, cudaMemcpyDeviceToHost, st));
+    uint32_t ctl[kCtlWords];
+    if ((s = fetch_ids(w, ids, (size_t)m * kstride, ctl, st)) != LQG_OK) return s;
+    return status_of(ctl);
 }
 
 }  // namespace lqg_host

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -47,37 +48,14 @@ enum : int {
     kCtlLatencyCount = kCtlFlagged
 };
 constexpr int kCtlWords = 8;
+// Ids of a host-buffer call that lie behind the control words in device memory, so
+// that one copy brings both: a copy to pageable memory costs the host 7 to 11 us
+// (37 queries of 200k x 96 with k 10, one B200: 9 us of 390), from about 64 KB on
+// copying the ids once more on the host costs that too.
+constexpr size_t kNearIds = 16384;
 
 constexpr uint32_t kMaxEf = 512;
 constexpr uint32_t kHeapGlobalCap = 28672;  // heap kernel search-pool slots in global memory
-
-// Pinned staging for copies between pageable host buffers and the device: four
-// slots, so that the host copies one while the copy engine moves the others.
-// 16 KB slots serve calls of a few queries (pinning 2 MB takes 3 ms), the first
-// larger copy brings 512 KB ones. Buffers that the caller pinned are copied
-// directly. The control words of a batch have a place of their own.
-// (One B200, 37 queries of 200k x 96: 489 -> 473 us per call; one FastScan query
-// 272 -> 241 us, with the batch's control words reset by one launch.)
-struct HostStage {
-    static constexpr size_t kSmall = 16 * 1024, kLarge = 512 * 1024;
-    static constexpr int kSlots = 4;
-    size_t slot = 0;
-    unsigned char* p = nullptr;  // slots, then the control words
-    cudaEvent_t ev[kSlots] = {};
-    bool busy[kSlots] = {};      // a host-to-device copy may still read the slot
-    int next = 0;
-    uint32_t* ctl() const { return reinterpret_cast<uint32_t*>(p + kSlots * slot); }
-    void release() {
-        for (auto& e : ev) {
-            if (e) cudaEventDestroy(e);
-            e = nullptr;
-        }
-        for (auto& b : busy) b = false;
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        slot = 0;
-    }
-};
 
 // Mutable device state of one batch in flight: control words, the list of
 // tie-flagged queries, the exact kernel's work areas, and staging buffers for
@@ -115,9 +93,11 @@ struct Workspace {
     // the call
     unsigned char* h_plain = nullptr;
     size_t cap_h_plain = 0;
-    HostStage stage;
+    // host-buffer calls: where few ids arrive together with the control words
+    uint32_t* h_near = nullptr;
     void release() {
-        stage.release();
+        std::free(h_near);
+        h_near = nullptr;
         if (h_plain) cudaFreeHost(h_plain);
         h_plain = nullptr;
         cap_h_plain = 0;
@@ -198,14 +178,14 @@ lqg_status grow(T*& p, size_t& cap, size_t need) {
     return LQG_OK;
 }
 
-// Copies through w.stage (host_stage.cu). copy_in returns when src may be
-// reused; copy_out when dst holds the data; fetch_ctl requests the batch's
-// control words, which w.stage.ctl() holds once a later copy_out has returned
-// (`most`: the most bytes of the copies that follow, so that none of them
-// replaces the staging).
-lqg_status copy_in(Workspace& w, void* dst, const void* src, size_t n, cudaStream_t st);
-lqg_status copy_out(Workspace& w, void* dst, const void* src, size_t n, cudaStream_t st);
-lqg_status fetch_ctl(Workspace& w, size_t most, cudaStream_t st);
+// Where the n ids of a host-buffer call go on the device (after ensure_ctl), and
+// their copy to the host, with the batch's control words; the latter waits.
+// Pageable memory is copied as it is: pinned staging of the library's own was no
+// faster (5 MB in and out of the device 345 and 339 us through four slots of
+// 512 KB, 283 and 276 without), and pinning even 4 KB takes 1.6 to 3 ms.
+lqg_status ids_area(Workspace& w, size_t n, uint32_t** area);
+lqg_status fetch_ids(Workspace& w, uint32_t* ids, size_t n, uint32_t (&ctl)[kCtlWords],
+                     cudaStream_t st);
 
 lqg_status ensure_ctl(Workspace& w, int64_t m);
 lqg_status ensure_exact(Workspace& w, int blocks, int warps_per_block);

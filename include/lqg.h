@@ -65,7 +65,15 @@ LQG_API void lqg_free(lqg_index* ix);
 /* Index.load: symqglib/qg/qg.hpp:217-224. The file must be exactly
  * 4 + 4*N*(D+deg) + N*D + 8*D bytes, optionally followed by a FastScan
  * section (see lqg_fs_build); every neighbour id must be < N.
- * Uploads the neighbour lists, codes and SQ8 parameters to the device. */
+ * Uploads the neighbour lists, codes and SQ8 parameters to the device.
+ *
+ * Device memory of an index (from lqg_load, lqg_set_arrays or a build):
+ * 4*N*deg bytes of lists, N*D (rows padded to 16) of codes, and, if they fit,
+ * 4*N*deg bytes of sums that spare most exact distances. When a later
+ * allocation of the library on that device finds no memory, the sums give way
+ * to it (the device is waited for; searches then return the same ids more
+ * slowly until the index gets new data), except sums that a captured graph of
+ * searches may read. */
 LQG_API lqg_status lqg_load(lqg_index* ix, const char* path);
 
 /* Index.save: symqglib/qg/qg.hpp:206-215 (same bytes). */

@@ -1010,6 +1010,46 @@ lqg_status fs_upload(lqg_index* ix) {
     return LQG_OK;
 }
 
+// Device rows and host copies of the codes and factors from the index's vectors.
+lqg_status fs_encode(lqg_index* ix) {
+    FsSection& f = ix->fs;
+    lqg_status s;
+    if ((s = fs_alloc(ix)) != LQG_OK) return s;
+    float* d_x = nullptr;
+    if ((s = fs_rows_base(ix, &d_x)) != LQG_OK) return s;
+    float* d_rot = nullptr;
+    uint32_t* d_nb = nullptr;
+    cudaError_t e = cudaMemcpy(f.d_diag, f.diag.data(), f.P * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && (cudaMalloc(&d_rot, ix->n * f.P * sizeof(float)) != cudaSuccess ||
+                             cudaMalloc(&d_nb, ix->n * ix->deg * sizeof(uint32_t)) != cudaSuccess)) {
+        cudaGetLastError();
+        cudaFree(d_x);
+        dfree(d_rot);
+        return fail(LQG_ERR_NOMEM, "FastScan encoder allocation failed");
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpy(d_nb, ix->nbrs.data(), ix->n * ix->deg * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        const int wpb = 4;
+        lqg::fs_rotate_kernel<<<8 * ix->num_sms, 32 * wpb, wpb * f.P * sizeof(float)>>>(
+            d_x, ix->n, ix->dim, f.P, f.d_diag, d_rot);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
+        lqg::fs_encode_kernel<<<16 * ix->num_sms, 256>>>(d_rot, d_nb, ix->n, f.P, ix->deg, f.d_rows,
+                                                         f.row_bytes, f.off_codes, f.off_fac);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    cudaFree(d_x);
+    cudaFree(d_rot);
+    cudaFree(d_nb);
+    if (e != cudaSuccess) return cuda_fail(e, "FastScan encoder");
+    if ((s = fs_download_packed(ix)) != LQG_OK) return s;
+    f.ready = true;
+    return LQG_OK;
+}
+
 lqg_status fs_check_batch(lqg_index* ix, const float* q, int64_t m, const uint32_t* k,
                           uint32_t k0, const uint32_t* ef, uint32_t& ef0, uint32_t* ids,
                           uint32_t kstride) {
@@ -1178,7 +1218,7 @@ lqg_status fs_read(lqg_index* ix, FILE* f) {
              std::fread(&fs.factors[i * 3 * ix->deg], 4, 3 * ix->deg, f) == 3 * ix->deg;
     }
     if (!ok) return fail(LQG_ERR_IO, "short read of the FastScan section");
-    return fs_upload(ix);
+    return with_sums_in_reserve(ix, [&] { return fs_upload(ix); });
 }
 
 lqg_status fs_write(const lqg_index* ix, FILE* f) {
@@ -1213,41 +1253,7 @@ LQG_API lqg_status lqg_fs_build(lqg_index* ix, uint64_t seed) {
     std::mt19937_64 gen(seed);
     const float sc = 1.0f / std::sqrt((float)f.P);
     for (uint32_t i = 0; i < f.P; ++i) f.diag[i] = (gen() & 1) ? sc : -sc;
-    lqg_status s;
-    if ((s = fs_alloc(ix)) != LQG_OK) return s;
-    float* d_x = nullptr;
-    if ((s = fs_rows_base(ix, &d_x)) != LQG_OK) return s;
-    float* d_rot = nullptr;
-    uint32_t* d_nb = nullptr;
-    cudaError_t e = cudaMemcpy(f.d_diag, f.diag.data(), f.P * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && (cudaMalloc(&d_rot, ix->n * f.P * sizeof(float)) != cudaSuccess ||
-                             cudaMalloc(&d_nb, ix->n * ix->deg * sizeof(uint32_t)) != cudaSuccess)) {
-        cudaGetLastError();
-        cudaFree(d_x);
-        dfree(d_rot);
-        return fail(LQG_ERR_NOMEM, "FastScan encoder allocation failed");
-    }
-    if (e == cudaSuccess)
-        e = cudaMemcpy(d_nb, ix->nbrs.data(), ix->n * ix->deg * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) {
-        const int wpb = 4;
-        lqg::fs_rotate_kernel<<<8 * ix->num_sms, 32 * wpb, wpb * f.P * sizeof(float)>>>(
-            d_x, ix->n, ix->dim, f.P, f.d_diag, d_rot);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) {
-        lqg::fs_encode_kernel<<<16 * ix->num_sms, 256>>>(d_rot, d_nb, ix->n, f.P, ix->deg, f.d_rows,
-                                                         f.row_bytes, f.off_codes, f.off_fac);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    cudaFree(d_x);
-    cudaFree(d_rot);
-    cudaFree(d_nb);
-    if (e != cudaSuccess) return cuda_fail(e, "FastScan encoder");
-    if ((s = fs_download_packed(ix)) != LQG_OK) return s;
-    f.ready = true;
-    return LQG_OK;
+    return with_sums_in_reserve(ix, [&] { return fs_encode(ix); });
 }
 
 LQG_API lqg_status lqg_fs_set_arrays(lqg_index* ix, const float* diag, const uint8_t* packed,
@@ -1267,7 +1273,7 @@ LQG_API lqg_status lqg_fs_set_arrays(lqg_index* ix, const float* diag, const uin
     } catch (...) {
         return fail(LQG_ERR_NOMEM, "host allocation failed");
     }
-    return fs_upload(ix);
+    return with_sums_in_reserve(ix, [&] { return fs_upload(ix); });
 }
 
 LQG_API lqg_status lqg_fs_get_arrays(const lqg_index* ix, uint32_t* padded_dim, float* diag,
@@ -1290,8 +1296,10 @@ LQG_API lqg_status lqg_fs_search_batch_device(lqg_index* ix, const float* querie
     if (s != LQG_OK) return s;
     DeviceScope ds(ix->device);
     if (ds.err != cudaSuccess) return cuda_fail(ds.err, "cudaSetDevice");
-    return fs_run(ix, ix->ws, queries, m, k, k0, ef, ef0, ids, kstride, stats,
-                  (cudaStream_t)stream, false);
+    return with_sums_in_reserve(ix, [&] {
+        return fs_run(ix, ix->ws, queries, m, k, k0, ef, ef0, ids, kstride, stats,
+                      (cudaStream_t)stream, false);
+    });
 }
 
 LQG_API lqg_status lqg_fs_stream_status(lqg_index* ix, void* stream) {
@@ -1323,24 +1331,27 @@ LQG_API lqg_status lqg_fs_search_batch(lqg_index* ix, const float* queries, int6
             LQG_CUDA(cudaStreamCreateWithFlags(&ix->own_stream, cudaStreamNonBlocking));
         st = ix->own_stream;
     }
-    if ((s = grow(w.d_q, w.cap_q, (size_t)m * ix->dim)) != LQG_OK) return s;
-    uint32_t* d_ids = nullptr;
-    if ((s = ensure_ctl(w, 0)) != LQG_OK) return s;
-    if ((s = ids_area(w, (size_t)m * kstride, &d_ids)) != LQG_OK) return s;
-    if (k && (s = grow(w.d_kq, w.cap_kq, (size_t)m)) != LQG_OK) return s;
-    if (ef && (s = grow(w.d_efq, w.cap_efq, (size_t)m)) != LQG_OK) return s;
-    if (stats && (s = grow(w.d_stats, w.cap_stats, (size_t)m * 4)) != LQG_OK) return s;
-    LQG_CUDA(cudaMemcpyAsync(w.d_q, queries, (size_t)m * ix->dim * 4, cudaMemcpyHostToDevice, st));
-    if (k) LQG_CUDA(cudaMemcpyAsync(w.d_kq, k, m * 4, cudaMemcpyHostToDevice, st));
-    if (ef) LQG_CUDA(cudaMemcpyAsync(w.d_efq, ef, m * 4, cudaMemcpyHostToDevice, st));
-    s = fs_run(ix, w, w.d_q, m, k ? w.d_kq : nullptr, k0, ef ? w.d_efq : nullptr, efb, d_ids,
-               kstride, stats ? w.d_stats : nullptr, st, m == 1);
-    if (s != LQG_OK) return s;
-    if (stats)
-        LQG_CUDA(cudaMemcpyAsync(stats, w.d_stats, (size_t)m * 16, cudaMemcpyDeviceToHost, st));
-    uint32_t ctl[kCtlWords];
-    if ((s = fetch_ids(w, ids, (size_t)m * kstride, ctl, st)) != LQG_OK) return s;
-    return fs_status_of(ctl);
+    return with_sums_in_reserve(ix, [&]() -> lqg_status {
+        lqg_status s;
+        if ((s = grow(w.d_q, w.cap_q, (size_t)m * ix->dim)) != LQG_OK) return s;
+        uint32_t* d_ids = nullptr;
+        if ((s = ensure_ctl(w, 0)) != LQG_OK) return s;
+        if ((s = ids_area(w, (size_t)m * kstride, &d_ids)) != LQG_OK) return s;
+        if (k && (s = grow(w.d_kq, w.cap_kq, (size_t)m)) != LQG_OK) return s;
+        if (ef && (s = grow(w.d_efq, w.cap_efq, (size_t)m)) != LQG_OK) return s;
+        if (stats && (s = grow(w.d_stats, w.cap_stats, (size_t)m * 4)) != LQG_OK) return s;
+        LQG_CUDA(cudaMemcpyAsync(w.d_q, queries, (size_t)m * ix->dim * 4, cudaMemcpyHostToDevice, st));
+        if (k) LQG_CUDA(cudaMemcpyAsync(w.d_kq, k, m * 4, cudaMemcpyHostToDevice, st));
+        if (ef) LQG_CUDA(cudaMemcpyAsync(w.d_efq, ef, m * 4, cudaMemcpyHostToDevice, st));
+        s = fs_run(ix, w, w.d_q, m, k ? w.d_kq : nullptr, k0, ef ? w.d_efq : nullptr, efb, d_ids,
+                   kstride, stats ? w.d_stats : nullptr, st, m == 1);
+        if (s != LQG_OK) return s;
+        if (stats)
+            LQG_CUDA(cudaMemcpyAsync(stats, w.d_stats, (size_t)m * 16, cudaMemcpyDeviceToHost, st));
+        uint32_t ctl[kCtlWords];
+        if ((s = fetch_ids(w, ids, (size_t)m * kstride, ctl, st)) != LQG_OK) return s;
+        return fs_status_of(ctl);
+    });
 }
 
 LQG_API lqg_status lqg_selftest_bounded_wait(int device, uint32_t tries, uint32_t* timed_out) {

@@ -3,6 +3,9 @@
 // esum[i][j] = nsum[nbrs[i][j]], so that a popped node's list brings its
 // neighbours' sums in the same coalesced read as their ids (a gather per
 // neighbour would cost a 32-byte sector each).
+#include <algorithm>
+#include <mutex>
+
 #include "lqg_host.h"
 #include "lqg_internal.h"
 
@@ -65,6 +68,52 @@ __global__ void repeated_id_kernel(const uint32_t* __restrict__ nbrs, uint64_t n
 
 namespace lqg_host {
 
+namespace {
+
+// The indexes that hold sums. Lock order: the list, then an index's sums.
+struct Holders {
+    std::mutex mu;
+    std::vector<lqg_index*> list;
+};
+Holders& holders() {
+    static Holders* h = new Holders;  // outlives every index
+    return *h;
+}
+
+// Frees ix's sums; with the list and the sums locked.
+void free_sums(Holders& h, lqg_index* ix) {
+    dfree(ix->d_nsum);
+    dfree(ix->d_esum);
+    ix->captured = false;
+    h.list.erase(std::remove(h.list.begin(), h.list.end(), ix), h.list.end());
+}
+
+}  // namespace
+
+void drop_sums(lqg_index* ix) {
+    Holders& h = holders();
+    std::lock_guard<std::mutex> lk(h.mu);
+    std::unique_lock<std::shared_mutex> l(ix->sums_mu);
+    free_sums(h, ix);
+}
+
+bool give_back_sums(lqg_index* ix) {
+    Holders& h = holders();
+    std::lock_guard<std::mutex> lk(h.mu);
+    lqg_index* from = nullptr;  // its own rather than another's
+    for (lqg_index* x : h.list)
+        if (x->device == ix->device && !x->captured && (!from || x == ix)) from = x;
+    if (!from) return false;
+    DeviceScope ds(from->device);
+    std::unique_lock<std::shared_mutex> l(from->sums_mu);  // no further call reads them
+    if (from->captured || ds.err != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    free_sums(h, from);
+    return true;
+}
+
 lqg_status check_distinct(lqg_index* ix, cudaStream_t st) {
     ix->distinct = 0;
     uint32_t* d = nullptr;
@@ -87,6 +136,7 @@ lqg_status check_distinct(lqg_index* ix, cudaStream_t st) {
 }
 
 lqg_status filter_node_sums(lqg_index* ix, cudaStream_t st) {
+    std::shared_lock<std::shared_mutex> lk(ix->sums_mu);
     if (!ix->d_nsum || !ix->d_esum) return LQG_OK;
     lqg::node_sum_kernel<<<8 * ix->num_sms, 256, 0, st>>>(ix->d_codes, ix->d_params, ix->n, ix->dim,
                                                           ix->cstride, ix->d_nsum);
@@ -95,6 +145,7 @@ lqg_status filter_node_sums(lqg_index* ix, cudaStream_t st) {
 }
 
 lqg_status filter_edge_sums(lqg_index* ix, cudaStream_t st) {
+    std::shared_lock<std::shared_mutex> lk(ix->sums_mu);
     if (!ix->d_nsum || !ix->d_esum) return LQG_OK;
     lqg::edge_sum_kernel<<<8 * ix->num_sms, 256, 0, st>>>(ix->d_nbrs, ix->d_nsum,
                                                           ix->n * ix->deg, ix->d_esum);
@@ -103,14 +154,25 @@ lqg_status filter_edge_sums(lqg_index* ix, cudaStream_t st) {
 }
 
 void filter_alloc(lqg_index* ix) {
-    dfree(ix->d_nsum);
-    dfree(ix->d_esum);
-    if (cudaMalloc(&ix->d_nsum, ix->n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&ix->d_esum, ix->n * ix->deg * sizeof(float)) != cudaSuccess) {
-        cudaGetLastError();
-        dfree(ix->d_nsum);
-        dfree(ix->d_esum);
+    Holders& h = holders();
+    std::lock_guard<std::mutex> lk(h.mu);
+    std::unique_lock<std::shared_mutex> l(ix->sums_mu);
+    free_sums(h, ix);
+    try {
+        h.list.push_back(ix);
+    } catch (...) {
+        return;  // no room for the list: no sums
     }
+    if (cudaMalloc(&ix->d_nsum, ix->n * sizeof(float)) == cudaSuccess &&
+        cudaMalloc(&ix->d_esum, ix->n * ix->deg * sizeof(float)) == cudaSuccess)
+        return;
+    cudaGetLastError();
+    free_sums(h, ix);
+}
+
+void filter_done(lqg_index* ix) {
+    std::unique_lock<std::shared_mutex> lk(ix->sums_mu);
+    dfree(ix->d_nsum);
 }
 
 }  // namespace lqg_host

@@ -65,6 +65,8 @@ lqg_status validate_content(const lqg_index* ix) {
 lqg_status upload(lqg_index* ix) {
     DeviceScope ds(ix->device);
     if (ds.err != cudaSuccess) return cuda_fail(ds.err, "cudaSetDevice");
+    ix->has_data = false;
+    drop_sums(ix);
     dfree(ix->d_nbrs);
     dfree(ix->d_codes);
     dfree(ix->d_params);
@@ -88,6 +90,7 @@ lqg_status upload(lqg_index* ix) {
     if ((s = filter_node_sums(ix, nullptr)) != LQG_OK) return s;
     if ((s = filter_edge_sums(ix, nullptr)) != LQG_OK) return s;
     if ((s = check_distinct(ix, nullptr)) != LQG_OK) return s;
+    filter_done(ix);
     ix->has_data = true;
     return LQG_OK;
 }
@@ -204,12 +207,14 @@ lqg::ShapeIndex shape_index(const lqg_index* ix) {
 
 // Fast kernel over all queries, then the exact kernel over the flagged ones.
 // `plain` launches one warp (the one-query-per-launch form).
-lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
-    lqg_status s = check_batch(ix, b);
-    if (s != LQG_OK) return s;
-    if (b.m == 0) return LQG_OK;
-    DeviceScope ds(ix->device);
-    if (ds.err != cudaSuccess) return cuda_fail(ds.err, "cudaSetDevice");
+static lqg_status run_checked(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
+    lqg_status s;
+    std::shared_lock<std::shared_mutex> sums(ix->sums_mu);
+    if (!plain) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(b.st, &cs) != cudaSuccess) cudaGetLastError();
+        if (cs != cudaStreamCaptureStatusNone) ix->captured = true;
+    }
     if ((s = ensure_ctl(w, b.m)) != LQG_OK) return s;
     if ((s = ensure_exact(w, ix->num_sms, 4)) != LQG_OK) return s;
     if ((s = reset_ctl(w, b.st)) != LQG_OK) return s;
@@ -511,6 +516,15 @@ lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
     return LQG_OK;
 }
 
+lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain) {
+    lqg_status s = check_batch(ix, b);
+    if (s != LQG_OK) return s;
+    if (b.m == 0) return LQG_OK;
+    DeviceScope ds(ix->device);
+    if (ds.err != cudaSuccess) return cuda_fail(ds.err, "cudaSetDevice");
+    return with_sums_in_reserve(ix, [&] { return run_checked(ix, w, b, plain); });
+}
+
 // The status of a finished batch from its control words.
 lqg_status status_of(const uint32_t* ctl) {
     if (ctl[kCtlErr]) {
@@ -699,7 +713,7 @@ lqg_status lqg_load(lqg_index* ix, const char* path) {
         return fail(LQG_ERR_IO, std::string("short read from ") + path);
     }
     lqg_status s = validate_content(ix);
-    if (s == LQG_OK) s = upload(ix);
+    if (s == LQG_OK) s = with_sums_in_reserve(ix, [&] { return upload(ix); });
     if (s == LQG_OK && with_fs) s = fs_read(ix, f);
     std::fclose(f);
     return s;
@@ -746,7 +760,7 @@ lqg_status lqg_set_arrays(lqg_index* ix, uint32_t entry, const float* vectors,
     ix->fs.release();  // the graph changed: its FastScan section is stale
     lqg_status s = validate_content(ix);
     if (s != LQG_OK) return s;
-    return upload(ix);
+    return with_sums_in_reserve(ix, [&] { return upload(ix); });
 }
 
 lqg_status lqg_get_arrays(const lqg_index* ix, uint32_t* entry, float* vectors, uint32_t* nbrs,
@@ -776,8 +790,11 @@ lqg_status lqg_search(lqg_index* ix, const float* query, uint32_t k, uint32_t* r
     if (!ix->own_stream) LQG_CUDA(cudaStreamCreateWithFlags(&ix->own_stream, cudaStreamNonBlocking));
     lqg_status s;
     Workspace& w = ix->ws;
-    if ((s = grow(w.d_q, w.cap_q, ix->dim)) != LQG_OK) return s;
-    if ((s = grow(w.d_ids, w.cap_ids, k)) != LQG_OK) return s;
+    s = with_sums_in_reserve(ix, [&] {
+        const lqg_status g = grow(w.d_q, w.cap_q, ix->dim);
+        return g != LQG_OK ? g : grow(w.d_ids, w.cap_ids, k);
+    });
+    if (s != LQG_OK) return s;
     cudaStream_t st = ix->own_stream;
     // pinned staging: query | ids | control words, each on 16 bytes
     const size_t qb = ((size_t)ix->dim * 4 + 15) & ~(size_t)15;
@@ -843,8 +860,10 @@ lqg_status lqg_search_batch(lqg_index* ix, const float* queries, int64_t m, cons
     if (k)
         for (int64_t i = 0; i < m; ++i)
             if (k[i] > kstride) return fail(LQG_ERR_ARG, "k exceeds kstride");
-    return search_host(ix, ix->ws, queries, m, k, k0, ef, efb, ids, kstride, pool_ids, pool_d,
-                       pstride, stats, st);
+    return with_sums_in_reserve(ix, [&] {
+        return search_host(ix, ix->ws, queries, m, k, k0, ef, efb, ids, kstride, pool_ids, pool_d,
+                           pstride, stats, st);
+    });
 }
 
 lqg_status lqg_search_exact_device(lqg_index* ix, const float* queries, int64_t m,
@@ -860,8 +879,11 @@ lqg_status lqg_search_exact_device(lqg_index* ix, const float* queries, int64_t 
     DeviceScope ds(ix->device);
     if (ds.err != cudaSuccess) return cuda_fail(ds.err, "cudaSetDevice");
     Workspace& w = ix->ws;
-    if ((s = ensure_ctl(w, 1)) != LQG_OK) return s;
-    if ((s = ensure_exact(w, ix->num_sms, 4)) != LQG_OK) return s;
+    s = with_sums_in_reserve(ix, [&] {
+        const lqg_status g = ensure_ctl(w, 1);
+        return g != LQG_OK ? g : ensure_exact(w, ix->num_sms, 4);
+    });
+    if (s != LQG_OK) return s;
     if ((s = reset_ctl(w, b.st)) != LQG_OK) return s;
     SearchArgs x = base_args(ix, w, b);
     x.qhead = w.d_ctl + kCtlExactHead;
@@ -1017,8 +1039,7 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
     dfree(ix->d_nbrs);
     dfree(ix->d_codes);
     dfree(ix->d_params);
-    dfree(ix->d_nsum);
-    dfree(ix->d_esum);
+    drop_sums(ix);
     ix->distinct = 0;
 
     const uint32_t rest_stride = 64, rev_cap = deg;
@@ -1050,10 +1071,10 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
         ix->tune = saved_tune;
     };
     auto alloc = [&](auto*& p, size_t bytes) {
-        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        while (cudaMalloc(&p, bytes) != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
-            return false;
+            if (!give_back_sums(ix)) return false;  // another index's
         }
         return true;
     };
@@ -1129,7 +1150,8 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
     ix->fs.release();  // a new graph: any FastScan section is stale
 
     for (uint32_t it = 0; it < num_iter; ++it) {
-        if ((s = filter_edge_sums(ix, st)) != LQG_OK || (s = check_distinct(ix, st)) != LQG_OK) {
+        if ((s = filter_edge_sums(ix, st)) != LQG_OK ||
+            (s = with_sums_in_reserve(ix, [&] { return check_distinct(ix, st); })) != LQG_OK) {
             cleanup();
             return s;
         }
@@ -1202,10 +1224,12 @@ lqg_status lqg_build_ex(lqg_index* ix, const float* data, uint32_t ef_build, uin
         LQG_BCUDA(lqg::launch_random_fill(d_new, d_new_cnt, n, deg, seed + 1 + it, st), "fill");
         LQG_BCUDA(cudaMemcpy(ix->d_nbrs, d_new, n * deg * 4, cudaMemcpyDeviceToDevice), "graph");
     }
-    if ((s = filter_edge_sums(ix, st)) != LQG_OK || (s = check_distinct(ix, st)) != LQG_OK) {
+    if ((s = filter_edge_sums(ix, st)) != LQG_OK ||
+        (s = with_sums_in_reserve(ix, [&] { return check_distinct(ix, st); })) != LQG_OK) {
         cleanup();
         return s;
     }
+    filter_done(ix);
     LQG_BCUDA(cudaMemcpy(ix->nbrs.data(), ix->d_nbrs, n * deg * 4, cudaMemcpyDeviceToHost), "graph");
     LQG_BCUDA(cudaMemcpy2D(ix->codes.data(), dim, ix->d_codes, ix->cstride, dim, n,
                            cudaMemcpyDeviceToHost), "codes");

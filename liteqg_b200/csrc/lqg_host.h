@@ -5,8 +5,10 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -213,6 +215,8 @@ struct FsSection {
     }
 };
 
+void drop_sums(lqg_index* ix);
+
 }  // namespace lqg_host
 
 struct lqg_index {
@@ -233,9 +237,13 @@ struct lqg_index {
     uint8_t* d_codes = nullptr;
     float* d_params = nullptr;
     // sums of the integer distance bound (filter.cu); NULL when they did not
-    // fit in device memory (the kernels then evaluate every candidate)
-    float* d_nsum = nullptr;  // [n]
+    // fit in device memory (the kernels then evaluate every candidate). Only a
+    // reserve: while no call reads them (sums_mu held alone) and no captured
+    // graph does, another allocation may take their place.
+    float* d_nsum = nullptr;  // [n], while the lists may change
     float* d_esum = nullptr;  // [n][deg]
+    std::shared_mutex sums_mu;
+    std::atomic<bool> captured{false};  // a call that reads them was captured
     uint32_t distinct = 0;    // no neighbour list holds an id twice
 
     lqg_host::Workspace ws;  // the default work area (one batch at a time)
@@ -254,8 +262,7 @@ struct lqg_index {
         lqg_host::dfree(d_nbrs);
         lqg_host::dfree(d_codes);
         lqg_host::dfree(d_params);
-        lqg_host::dfree(d_nsum);
-        lqg_host::dfree(d_esum);
+        lqg_host::drop_sums(this);
         ws.release();
         fs.release();
         if (own_stream) cudaStreamDestroy(own_stream);
@@ -267,8 +274,19 @@ namespace lqg_host {
 lqg_status check_batch(lqg_index* ix, BatchSpec& b);
 lqg_status run_batch(lqg_index* ix, Workspace& w, BatchSpec& b, bool plain);
 // Sums of the integer distance bound (filter.cu): buffers, per-node sums of
-// the current codes, per-slot sums of the current lists.
+// the current codes, per-slot sums of the current lists; no further lists.
 void filter_alloc(lqg_index* ix);
+void filter_done(lqg_index* ix);
+// Gives the sums of `ix`, or else of another index on its device, back to the
+// device; false if none can go.
+bool give_back_sums(lqg_index* ix);
+// f(), again as long as it finds no device memory and sums can be given back.
+template <class F>
+lqg_status with_sums_in_reserve(lqg_index* ix, F f) {
+    lqg_status s = f();
+    while (s == LQG_ERR_NOMEM && give_back_sums(ix)) s = f();
+    return s;
+}
 // Whether any list of the index holds an id twice (sets ix->distinct; waits).
 lqg_status check_distinct(lqg_index* ix, cudaStream_t st);
 lqg_status filter_node_sums(lqg_index* ix, cudaStream_t st);

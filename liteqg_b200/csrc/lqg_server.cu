@@ -311,14 +311,7 @@ lqg_status warm_context(lqg_server* s, Ctx& c) {
     return LQG_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-lqg_status lqg_server_start(lqg_index* ix, const lqg_server_config* cfg, lqg_server** out) {
-    if (!ix || !out) return fail(LQG_ERR_ARG, "null argument");
-    *out = nullptr;
-    if (!ix->has_data) return fail(LQG_ERR_STATE, "index has no data");
+lqg_status server_start(lqg_index* ix, const lqg_server_config* cfg, lqg_server** out) {
     lqg_server_config c = cfg ? *cfg : lqg_server_config{};
     if (c.streams == 0) c.streams = 4;
     if (c.max_k == 0) c.max_k = 100;
@@ -383,6 +376,17 @@ lqg_status lqg_server_start(lqg_index* ix, const lqg_server_config* cfg, lqg_ser
     s->completer = std::thread(complete_loop, s);
     *out = s;
     return LQG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+lqg_status lqg_server_start(lqg_index* ix, const lqg_server_config* cfg, lqg_server** out) {
+    if (!ix || !out) return fail(LQG_ERR_ARG, "null argument");
+    *out = nullptr;
+    if (!ix->has_data) return fail(LQG_ERR_STATE, "index has no data");
+    return with_sums_in_reserve(ix, [&] { return server_start(ix, cfg, out); });
 }
 
 lqg_status lqg_server_submit(lqg_server* s, const float* query, uint32_t k, uint32_t ef,

@@ -8,6 +8,53 @@ from oracle.oracle import IndexArrays, Oracle, sq8_quantize
 pytestmark = pytest.mark.gpu
 
 
+# With a bound on ef of 200 and more, the latency form's blocks have room for a larger
+# visited cache than the one-warp form's 2,048 slots. The latter forgets nodes, and
+# evaluates again those that overlapping lists name again: a query's evaluation count
+# tells which form ran it. On B200 the latency form has 1,184 blocks
+# at 48 dimensions and degree 32. More than 8,192 queries at ef 512 go in chunks of
+# 8,192, each with a choice of its own.
+@pytest.mark.parametrize("m,top,long_ones,forms", [
+    (3001, 200, 60, ["latency"]),            # few long queries
+    (3001, 200, 1, ["latency"]),
+    (3001, 200, 3001, ["warp"]),             # all the same
+    (12000, 200, 12000, ["warp"]),
+    (20000, 200, 60, ["warp"]),              # past 16 per block: no look at all
+    (10192, 512, 40, ["latency", "warp"]),   # the long ones in the first chunk
+])
+def test_the_form_that_runs(m, top, long_ones, forms):
+    import liteqg_b200
+
+    rng = np.random.default_rng(m + long_ones)
+    n, dim, deg, k, chunk = 30000, 48, 32, 5, 8192 if top == 512 else m
+    x = rng.integers(0, 24, (n, dim)).astype(np.float32)
+    q = rng.integers(0, 24, (m, dim)).astype(np.float32)
+    ef = np.full(m, 16, np.uint32)
+    ef[rng.choice(chunk, long_ones, replace=False)] = top
+    ring = (np.arange(n)[:, None] + np.r_[-14:0, 1:15, rng.integers(15, n - 15, 4)]) % n
+    ids = rng.permutation(n)
+    nb = np.empty((n, deg), np.int64)
+    nb[ids] = ids[ring]
+    codes, params = sq8_quantize(x, 2)
+    ix = liteqg_b200.Index("QG", "L2", n, dim, deg)
+    ix.set_arrays(7, x, nb.astype(np.uint32), codes, params)
+    ids, st = ix.search(q, k, ef=ef, return_stats=True)
+    ix.set_tuning(small_batch=0xFFFFFFFF)
+    warp_ids, warp = ix.search(q, k, ef=ef, return_stats=True)
+    ix.set_tuning(small_batch=1 << 20)
+    latency_ids, latency = ix.search(q, k, ef=ef, return_stats=True)
+    assert np.array_equal(ids, warp_ids) and np.array_equal(ids, latency_ids)
+    for c, form in enumerate(forms):
+        rows = slice(c * chunk, (c + 1) * chunk)
+        want, other = (warp, latency) if form == "warp" else (latency, warp)
+        assert np.array_equal(st[rows], want[rows]), form
+        assert not np.array_equal(st[rows], other[rows]), form
+    oracle = Oracle(IndexArrays(n, dim, deg, 7, x, nb.astype(np.uint32), codes, params))
+    for e in np.unique(ef):
+        rows = np.concatenate([np.flatnonzero(ef == e)[:40], np.flatnonzero(ef == e)[-40:]])
+        assert np.array_equal(ids[rows], oracle.search(q[rows], k, int(e)).compat)
+
+
 def test_capture_with_ef_after_a_call_without():
     """After one eager call of a size, a call of that size allocates nothing,
     whether or not it has a per-query ef: it can be captured."""

@@ -1079,7 +1079,7 @@ def uneven_arm(args, w, name, device):
     best = None
     # (mode, lanes per candidate, heap warps per block, heap slots, visited
     # bits[, 1: batch kernels one query per block])
-    shapes = ((6, 2, 4, 512, 10), (6, 4, 4, 512, 10), (5, 2, 4, 512, 10), (4, 4, 4, 512, 10),
+    shapes = ((6, 2, 4, 512, 10), (5, 2, 4, 512, 10), (4, 4, 4, 512, 10),
               (2, 2, 4, 512, 10), (2, 4, 4, 512, 10), (1, 4, 4, 512, 10),
               (2, 2, 4, 256, 10), (2, 2, 4, 256, 9), (2, 2, 2, 512, 10), (2, 2, 8, 256, 9),
               # larger visited caches: fewer forgotten nodes evaluated again at
@@ -1215,7 +1215,7 @@ def uneven_arm(args, w, name, device):
                                f"per-query ef from {list(w['ef_choices'])}, k from "
                                f"{list(w['k_choices'])} (seed 2)",
                    "recall_at_10_pool_by_ef": rec_by_ef, "pool_coverage_at_10_by_ef": cov_by_ef,
-                   "mode": best[1], "lanes_per_cand": 4 if best[6] else best[2],
+                   "mode": best[1], "lanes_per_cand": 8 if best[1] >= 5 else best[2],
                    "warps_per_block": 4 if best[6] else best[3], "heap_scap": best[4],
                    "visited_bits": best[5], "query_per_block": best[6],
                    "l2": "flushed between steps (256 MiB write)"},
@@ -1351,7 +1351,7 @@ def serving_arm(args, w, name, device):
                                f"{list(w['ef_choices'])}", "recall_at_10_pool_by_ef": rec,
                    "pool_coverage_at_10_by_ef": cov,
                    "server": {"streams": SERVING_STREAMS, "mode": best[1],
-                              "lanes_per_cand": best[2]}},
+                              "lanes_per_cand": 8 if best[1] >= 5 else best[2]}},
         "serving": rows,
         "plain_qps": len(lat) / sum(lat), "plain_p50_ms": 1e3 * float(np.percentile(lat, 50)),
         "plain_p99_ms": 1e3 * float(np.percentile(lat, 99)),

@@ -17,21 +17,17 @@ import numpy as np
 
 DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "liteqg_b200", "tuning.json")
 
-# (mode, lanes_per_cand, visited_bits, warps_per_block, heap_warps, heap_scap)
+# (mode, lanes_per_cand, visited_bits, warps_per_block, heap_warps, heap_scap);
+# modes 5 and 6 run the same whatever the lanes
 CANDIDATES = [
     (6, 2, 10, 8, 4, 256),
-    (6, 4, 10, 8, 4, 256),
     (6, 2, 10, 8, 5, 256),
-    (6, 4, 10, 8, 5, 256),
     (6, 2, 10, 8, 4, 512),
     (6, 2, 9, 8, 5, 256),
     (5, 2, 10, 8, 4, 256),
-    (5, 4, 10, 8, 4, 256),
     (5, 2, 10, 8, 4, 512),
-    (5, 4, 10, 8, 4, 512),
     (5, 2, 11, 8, 4, 512),
     (5, 2, 10, 8, 5, 256),
-    (5, 4, 10, 8, 5, 256),
     (4, 2, 10, 8, 4, 256),
     (4, 2, 10, 8, 4, 512),
     (4, 4, 10, 8, 4, 512),

@@ -221,8 +221,9 @@ LQG_API lqg_status lqg_search_exact_noalloc(lqg_index* ix, const float* queries,
 /* Launch shape and policy. 0 fields keep the current value. A new index
  * starts with mode 6, lanes_per_cand 2, visited_bits 10, warps_per_block 8,
  * heap_warps 4, heap_scap 256.
- *   lanes_per_cand  {1,2,4,8,16}: lanes sharing one distance (modes 1-4;
- *                   modes 5-6 take 2, 4 or 8 and always use 4)
+ *   lanes_per_cand  {1,2,4,8,16}: lanes sharing one distance in the heap, replay
+ *                   and split kernels (modes 1-4; the fast kernel and modes 5-6
+ *                   always use 8)
  *   visited_bits    [8, 13]: size of the per-query visited cache (4 * 2^bits
  *                   bytes; modes 5-6 hold 2^(bits+1) 16-bit slots, the others
  *                   2^bits ids). At the default of 10, modes 5-6 take a larger

@@ -315,10 +315,6 @@ static lqg_status run_checked(lqg_index* ix, Workspace& w, BatchSpec& b, bool pl
             ra.scap = lqg::batch_heap_slots(shape, h.vbits, ra.scap, ra.acap, sw);
         }
         if (cta) sw = 1;
-        // the batch kernels' distance passes use 4 lanes per candidate; the
-        // tuning field keeps its accepted values
-        if (batch && !cta && t.lanes_per_cand != 2 && t.lanes_per_cand != 4 && t.lanes_per_cand != 8)
-            return fail(LQG_ERR_ARG, "search kernel cannot launch with this tuning");
         auto launch = [&](const SearchArgs& c, int blocks, int* occ) {
             if (cta) return lqg::launch_batch_cta(c, ra, degw, blocks, b.st, occ);
             if (batch)

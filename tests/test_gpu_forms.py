@@ -90,3 +90,24 @@ def test_capture_with_ef_after_a_call_without():
         rows = np.flatnonzero(ef == e)[:60]
         assert np.array_equal(got[rows].view(np.uint32), oracle.search(q[rows], k, e).compat)
     del graph
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("mode", [5, 6])
+def test_lanes_do_not_matter(mode, lanes):
+    """The batch kernel has no use for lanes_per_cand: small and large batches run
+    with every value that set_tuning takes."""
+    import liteqg_b200
+
+    rng = np.random.default_rng(lanes)
+    n, dim, deg, k, ef = 1500, 48, 32, 10, 20
+    x = rng.integers(0, 24, (n, dim)).astype(np.float32)
+    nb = np.stack([rng.choice(n, deg, replace=False) for _ in range(n)]).astype(np.uint32)
+    codes, params = sq8_quantize(x, 2)
+    ix = liteqg_b200.Index("QG", "L2", n, dim, deg)
+    ix.set_arrays(7, x, nb, codes, params)
+    ix.set_tuning(mode=mode, lanes_per_cand=lanes)
+    oracle = Oracle(IndexArrays(n, dim, deg, 7, x, nb, codes, params))
+    for m in (1, 40, 4000):
+        q = rng.integers(0, 24, (m, dim)).astype(np.float32)
+        assert np.array_equal(ix.search(q, k, ef=ef)[-40:], oracle.search(q[-40:], k, ef).compat)

@@ -335,9 +335,10 @@ static lqg_status run_checked(lqg_index* ix, Workspace& w, BatchSpec& b, bool pl
         // longest-expected queries first, when a chunk holds more queries
         // than the launch has warps (otherwise they all start at once)
         const bool order = !plain && chunk > (int64_t)rb * sw;
-        // (with or without per-query ef: a batch of the same size that is captured
-        // later may have one, and allocates nothing)
-        if ((order || lblocks > 0) && (s = ensure_order(w, chunk)) != LQG_OK) return s;
+        // (also where a later batch of the same size may need a work list and must not
+        // allocate: one that is captured, with per-query ef after one without, and a
+        // server's batches, with per-query ef and the latency form only when alone)
+        if ((order || lblocks > 0 || (batch && b.efq)) && (s = ensure_order(w, chunk)) != LQG_OK) return s;
         const size_t slots = std::max((size_t)rb * sw, (size_t)lblocks);
         if (w.sp_global_slots < slots) {
             dfree(w.d_sp_global);

@@ -187,8 +187,8 @@ constexpr uint32_t kPairRedo = 16u; // the step's expansion does not count; expa
 // candidates of one pop, the others already expand the next (list and visited
 // cache by warp 1, then bound and exact distances over all of them, a segment of
 // the candidates each), with the bound from before the merge (it only falls, and
-// the merge tests every candidate again). One barrier per pop; candidates and
-// messages are double-buffered. Where the next pop is not certain - equal
+// the merge tests every candidate again). One barrier per pop, and one more among
+// three expanding warps; candidates and messages are double-buffered. Where the next pop is not certain - equal
 // smallest distances, or the search heap in use - the expanders wait a step for
 // warp 0 to pop. The nearest candidate can be a node that the visited cache forgot and
 // that was popped before. A table of the popped ids keeps most of them from being
@@ -205,16 +205,17 @@ constexpr uint32_t kPairRedo = 16u; // the step's expansion does not count; expa
 // and a small instruction footprint (loops over rows and members are not
 // unrolled: unrolled, instruction-cache misses took 20 % of the time).
 // Registers: 96 let 20 warps live on an SM without spills for rows below 256
-// bytes; 24 warps at 80 registers and fewer are slower (spills). Wider rows and
-// the query-per-block form are bound to fewer warps by shared memory, and take
-// 128.
-// Kernel time, before and after the distance bound, the list prefetch, the
-// checked-distinct lists and the 16-bit visited tags (one B200, us):
-//   1M x 128 deg 32 ef 64, 10,000 queries      2,818 -> 2,560
-//   200k x 96 deg 32 ef 100, 37 queries          600 ->   464
-//   100k x 768 deg 64 ef 128, 2,000 queries    4,930 -> 2,470
-//   100k x 960 deg 64 ef 32-512, 2,048        20,550 -> 10,970
-//   100k x 100 deg 96 ef 200, 1,777 queries    3,016 -> 2,334
+// bytes (but for 3 to 17 words at degree 32 to 128); 24 warps at 80 registers and
+// fewer are slower (spills). Wider rows and the latency form are bound to fewer
+// warps by shared memory, and take 128.
+// Device calls, before and after the distance bound, the list prefetch, the
+// checked-distinct lists, the 16-bit visited tags, the shorter heap steps and the
+// latency form's steps (one B200, us):
+//   1M x 128 deg 32 ef 64, 10,000 queries      2,932 -> 2,153
+//   200k x 96 deg 32 ef 100, 37 queries          577 ->   347
+//   100k x 768 deg 64 ef 128, 2,000 queries    4,750 -> 2,890
+//   100k x 960 deg 64 ef 32-512, 2,048        19,750 -> 6,370
+//   100k x 100 deg 96 ef 200, 1,777 queries    2,655 -> 1,825
 template <int DEGW, bool WIDE, int NE>
 __global__ void __maxnreg__(WIDE || NE ? kWideRegs : kNarrowRegs)
     batch_search_kernel(const __grid_constant__ SearchArgs a, const __grid_constant__ ReplayArgs ra) {

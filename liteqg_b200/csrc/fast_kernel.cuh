@@ -22,10 +22,11 @@
 //   distance) and is dropped. With lists of more than one 32-id word, equal
 //   distances of one expansion go by the candidates' places after the filter
 //   of a 2^vbits-slot cache of full ids (lane, then word), so that cache is
-//   kept too: it decides the places, the other one what is evaluated. Candidates are merged in ascending distance; any equality
-//   between a candidate and the pool, or between two candidates, with
-//   different ids (or a non-finite distance) hands the query to the exact
-//   kernel, since only there does the reference's heap layout decide.
+//   kept too: it decides the places, the other one what is evaluated.
+//   Candidates are merged in ascending distance; any equality between a
+//   candidate and the pool, or between two candidates, with different ids (or a
+//   non-finite distance) hands the query to the exact kernel, since only there
+//   does the reference's heap layout decide.
 //
 // exact_search_kernel — one warp per query from a list. Emulates the
 //   reference literally: sp/rp as GCC libstdc++ binary heaps in global

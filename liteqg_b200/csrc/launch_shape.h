@@ -112,7 +112,7 @@ inline int batch_warps(const ShapeIndex& x, uint32_t acap, int warps, uint32_t& 
 // A larger cache forgets fewer nodes (at ef 200 and degree 96: 10.5 k
 // evaluations per query at 10 bits, 6.5 k at 13, 5.6 k without forgetting), but
 // costs resident queries: a batch that fills the GPU runs at the tuned 10 bits
-// (1M x 128, 10,000 queries at ef 64: 2.75 ms at 10, 2.95 at 11, 4.45 at 12).
+// (1M x 128, 10,000 queries at ef 64: 2.15 ms at 10, 2.37 at 11, 3.30 at 12).
 // So a batch whose queries all fit at once takes the largest cache they fit
 // with, when the tuning field is at its default; other values are taken as they
 // are.
@@ -141,7 +141,7 @@ inline uint32_t batch_heap_slots(const ShapeIndex& x, uint32_t vbits, uint32_t s
 // plentiful: first room for the search heap of a query that meets a tie (past
 // its slots in shared memory a push waits for global memory: one tie cost a
 // query of 560 us another 350 at 256 slots), then the largest visited cache, up
-// to 2^14 (clearing it costs about 600 cycles per query).
+// to 14 bits (2^15 slots; clearing them costs about 600 cycles per query).
 inline void latency_shape(const ShapeIndex& x, int nb, uint32_t acap, uint32_t& vbits,
                           uint32_t& scap) {
     const size_t share = kSmBytes / nb / kBlockUnit * kBlockUnit;

@@ -212,8 +212,10 @@ static lqg_status run_checked(lqg_index* ix, Workspace& w, BatchSpec& b, bool pl
     std::shared_lock<std::shared_mutex> sums(ix->sums_mu);
     if (!plain) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(b.st, &cs) != cudaSuccess) cudaGetLastError();
-        if (cs != cudaStreamCaptureStatusNone) ix->captured = true;
+        if (cudaStreamIsCapturing(b.st, &cs) != cudaSuccess)
+            cudaGetLastError();  // (the legacy stream while another one captures)
+        else if (cs != cudaStreamCaptureStatusNone)
+            ix->captured = true;
     }
     if ((s = ensure_ctl(w, b.m)) != LQG_OK) return s;
     if ((s = ensure_exact(w, ix->num_sms, 4)) != LQG_OK) return s;

@@ -51,9 +51,10 @@ enum : int {
 };
 constexpr int kCtlWords = 8;
 // Ids of a host-buffer call that lie behind the control words in device memory, so
-// that one copy brings both: a copy to pageable memory costs the host 7 to 11 us
-// (37 queries of 200k x 96 with k 10, one B200: 9 us of 390), from about 64 KB on
-// copying the ids once more on the host costs that too.
+// that one copy brings both: a copy back to pageable memory costs 6 to 11 us (14 KB
+// in and 1.5 KB out around a kernel of 250 us, one B200: 274.9 us with two copies
+// back, 264.4 with one; 400 and 40 KB: 303 and 297). From about 64 KB on, copying
+// the ids once more on the host costs as much.
 constexpr size_t kNearIds = 16384;
 
 constexpr uint32_t kMaxEf = 512;
@@ -161,8 +162,8 @@ struct BatchSpec {
     uint32_t ties_ok = 0;
     uint32_t* path = nullptr;  // index build: popped ids per query (fast kernel)
     uint32_t path_stride = 0;
-    // the query-per-block form may run (modes 5-6, small batches): false when
-    // other batches share the device, where its idle helper warps would cost
+    // the latency form may run (modes 5-6, small batches): false when other
+    // batches share the device, where its few queries per SM would cost
     // throughput
     bool small_ok = true;
 };

@@ -42,10 +42,11 @@ __global__ void entry_distance_kernel(const float* __restrict__ q, int64_t m, ui
     }
 }
 
-// Which form of the batch kernel takes a batch of queries with an ef each: the latency form if its blocks can start all queries of more
-// than half of the largest ef at once and all queries together are the work of at
-// most 1.5 of the largest per block. (Such a batch ends when its longest queries do,
-// which the latency form finishes sooner, while the short ones leave blocks free.
+// Which form of the batch kernel takes a batch of queries with an ef each: the
+// latency form if its blocks can start all queries of more than half of the largest
+// ef at once and all queries together are the work of at most 1.5 of the largest per
+// block. (Such a batch ends when its longest queries do, which the latency form
+// finishes sooner, while the short ones leave blocks free.
 // us, one-warp against latency form, 100k vectors, k up to 100; ef 32 to 512 in
 // equal shares - at 960 dimensions and degree 64, 592 blocks: 1,184 queries 8040 and
 // 6402, 2,368 10081 and 7801, 3,552 10284 and 11287; at 128 and 32, 1,184 blocks:
@@ -53,8 +54,9 @@ __global__ void entry_distance_kernel(const float* __restrict__ q, int64_t m, ui
 // 888 queries 8473 and 9716; 1,776 at 128 dimensions 3206 and 3288.)
 // The latency form's work list is the queries by descending ef, counted into bins in
 // one block, in any order within a bin. (A batch that stays with the one-warp form
-// pays 10 to 16 us for this kernel and the other form's empty launch; with the sort
-// above in its place it was 50 to 70.)
+// pays 10 to 12 us for this kernel and the other form's empty launch up to 2,500
+// queries, 20 at 18,000: ef 10, 1,185 queries of 100k x 96 157 against 146 us; with
+// the sort above in its place it was 50 to 70.)
 __global__ void __launch_bounds__(1024) choose_form_kernel(const uint32_t* __restrict__ efq,
                                                            uint32_t m, uint32_t efmax,
                                                            uint32_t blocks, int32_t* list,

@@ -10,7 +10,8 @@
 //   y = sum (q - (min + s c))^2 = sum t^2 - sum g c + sum s^2 c^2,  g = 2 s t.
 // sum t^2 is per query, sum s^2 c^2 per node (stored per list slot, beside the
 // neighbour id: esum), and sum g c is an integer dot product once g is rounded
-// to 16 bits: g = st * G + r, G = 256 hi + lo with hi, lo in [-128, 127].
+// to 16 bits: g = st * G + r, G = 256 hi + lo with hi, lo in [-128, 127], so that
+// sum g c = st * sum G c + 128 sum r + sum r (c - 128).
 // mma.sync m16n8k32 (u8 x s8, exact 32-bit sums) takes 16 candidates by 32
 // dimensions against the two byte planes at once; the even columns hold hi,
 // the odd ones lo, so every lane of a row's quad ends with both sums. Lane
@@ -21,7 +22,7 @@
 // with 16 to 32 gathered rows per step.
 //
 // Error bound: A = K + S - st * dot differs from y by at most
-//   128 sum |r|          the rounding of g: |r| |c - 128|, with 128 sum r in K
+//   128 sum |r|          the rounding of g: |r| |c - 128|, with -128 sum r in K
 //   + 32 u M             every float rounding in K, S, st * dot and their sum,
 //                        u = 2^-24, M = K + sum (255 s)^2 + 256 sum |g|
 // and the reference's float distance y' (16 accumulators, at most 150
@@ -43,7 +44,7 @@ namespace lqg {
 constexpr float kFilterRel = 1.00004f;
 
 struct Sq8Filter {
-    float K;   // sum t^2 + 128 sum r
+    float K;   // sum t^2 - 128 sum r
     float st;  // step of G
     float E;   // absolute part of the bound
 };
@@ -92,7 +93,7 @@ __device__ __forceinline__ Sq8Filter filter_prepare(const float* qs, const float
             lo = ((G + 128) & 255) - 128;
             hi = (G - lo) >> 8;
             const float r = fmaf(-f.st, (float)G, g);
-            ks += (double)t * (double)t + 128.0 * (double)r;
+            ks += (double)t * (double)t - 128.0 * (double)r;
             R += fabsf(r);
             G1 += fabsf(g);
         }
